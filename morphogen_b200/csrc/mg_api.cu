@@ -876,7 +876,7 @@ int plan_warp(mg_batch* b, const std::vector<SegPlan>& segs, int G, uint32_t VT,
       items += (sp.keys.size() / sp.g) * ((nF + 31) / 32);
       slots = std::max(slots, M);
     }
-    uint32_t nw = (uint32_t)mg::kWarps;
+    uint32_t nw = mg::warp_cta_warps(G, VT);
     size_t smem = mg::warp_smem_bytes(G, VT, slots, nw);
     while (smem > ctx->smem_optin && nw > 4) {
       nw /= 2;
@@ -992,6 +992,9 @@ int plan_warp(mg_batch* b, const std::vector<SegPlan>& segs, int G, uint32_t VT,
         mg::warp_smem_bytes(G, VT, slots, 14) <= ctx->smem_optin)
       L.NW = 14;
   }
+  // Fewer items than the device has warps: CTAs just wide enough to spread
+  // them over all SMs, so that no scheduler holds two while another has none.
+  L.NW = (uint32_t)std::min<uint64_t>(L.NW, std::max<uint64_t>(1, (items + ctx->sms - 1) / ctx->sms));
   L.smem = mg::warp_smem_bytes(G, VT, slots, L.NW);
   if (int rc = prepare_warp(ctx, G, VT, L.smem)) return rc;
   const int occ = mg::warp_occupancy(G, VT, L.smem, L.NW);

@@ -6,9 +6,16 @@
 // rounds, feed-forward add, chacha_prg.rs:112-144).  Children: L = block0[0..4],
 // R = block0[4..8], tL = block1[0] & 1, tR = block1[1] & 1.
 //
-// B200 notes: the path is integer-ALU bound.  Adds and 3-input logic run at
-// the full 128 lanes/clk/SM, funnel shifts and byte permutes at half rate, so
-// the code is issue-bound at ~12 instructions per quarter round.  Both blocks
+// B200 notes: the path is bound by integer issue.  XOR/AND (LOP3), funnel
+// shifts (SHF) and byte permutes (PRMT) go to the ALU pipe and two-input adds
+// to the FMA pipe, both at 16 lanes per clock per scheduler, so a node
+// expansion written with one instruction per operation keeps the ALU pipe full
+// (456 instructions) and the FMA pipe half idle (227).  Rotations by 16 and 8
+// are whole bytes, and a byte-wise dot product plus a multiply-add does one on
+// the FMA pipe (rotl_bytes): with 69 of them there, 387 ALU and 366 FMA
+// instructions, 40.2 -> 44.6 G node expansions/s for the PRG alone
+// (mg_prg_peak).  More of them loses to the issue rate (one instruction per
+// clock and scheduler, 755 per expansion), fewer to the ALU pipe.  Both blocks
 // are written out in one straight-line function so the compiler shares the
 // three counter-independent column quarter rounds of round 1 and drops the
 // parts of block 1 that do not reach bit 0 of words 0 and 1.
@@ -60,56 +67,82 @@ struct alignas(16) KeyAux {
 };
 static_assert(sizeof(KeyAux) == 640, "KeyAux layout");
 
-__device__ __forceinline__ uint32_t rotl16(uint32_t x) { return __byte_perm(x, 0, 0x1032); }
-__device__ __forceinline__ uint32_t rotl8(uint32_t x) { return __byte_perm(x, 0, 0x2103); }
 __device__ __forceinline__ uint32_t rotl12(uint32_t x) { return __funnelshift_l(x, x, 12); }
 __device__ __forceinline__ uint32_t rotl7(uint32_t x) { return __funnelshift_l(x, x, 7); }
 
-#define MG_QR(a, b, c, d)              \
-  a += b; d ^= a; d = mg::rotl16(d);   \
-  c += d; b ^= c; b = mg::rotl12(b);   \
-  a += b; d ^= a; d = mg::rotl8(d);    \
-  c += d; b ^= c; b = mg::rotl7(b);
+// 2^16 and 2^8 read from constant memory: a multiplier the compiler cannot
+// see stays an integer multiply-add (with an immediate power of two it may
+// become a shift, which is back on the ALU pipe).
+static __constant__ uint32_t kRotMul[2] = {1u << 16, 1u << 8};
 
-#define MG_DOUBLE_ROUND(x)                                        \
-  MG_QR(x##0, x##4, x##8, x##12) MG_QR(x##1, x##5, x##9, x##13)   \
-  MG_QR(x##2, x##6, x##10, x##14) MG_QR(x##3, x##7, x##11, x##15) \
-  MG_QR(x##0, x##5, x##10, x##15) MG_QR(x##1, x##6, x##11, x##12) \
-  MG_QR(x##2, x##7, x##8, x##13) MG_QR(x##3, x##4, x##9, x##14)
+// rotl by 16 or 8, on the ALU pipe (one byte permute) or, with FMA set, as two
+// multiply-adds on the otherwise half-idle FMA pipe: the part shifted down is
+// a dot product with a one-hot byte vector (dp2a selects the upper half-word,
+// dp4a the top byte), and a multiply-add places the part shifted up above it.
+template <int N, bool FMA>
+__device__ __forceinline__ uint32_t rotl_bytes(uint32_t x) {
+  static_assert(N == 16 || N == 8, "whole bytes");
+  if constexpr (!FMA) return __byte_perm(x, 0, N == 16 ? 0x1032 : 0x2103);
+  const uint32_t down = N == 16 ? __dp2a_lo(x, 0x00000100u, 0u) : __dp4a(x, 0x01000000u, 0u);
+  return x * kRotMul[N == 16 ? 0 : 1] + down;
+}
 
-// ChaCha8Prg::expand.  tl/tr are 0 or 1.
+template <bool F16, bool F8>
+__device__ __forceinline__ void quarter_round(uint32_t& a, uint32_t& b, uint32_t& c, uint32_t& d) {
+  a += b; d ^= a; d = rotl_bytes<16, F16>(d);
+  c += d; b ^= c; b = rotl12(b);
+  a += b; d ^= a; d = rotl_bytes<8, F8>(d);
+  c += d; b ^= c; b = rotl7(b);
+}
+
+// Which of a block's rotations by 16 and 8 run on the FMA pipe (FMA set), by
+// round and quarter round: the 16s of quarter rounds 1..3 and the 8s of the
+// diagonal rounds, 69 of the 114 that matter.
+template <bool FMA, int RD, int C>
+__device__ __forceinline__ void qr_at(uint32_t& a, uint32_t& b, uint32_t& c, uint32_t& d) {
+  quarter_round<FMA && C != 0, FMA && (RD & 1) != 0>(a, b, c, d);
+}
+
+template <bool FMA, int DR>
+__device__ __forceinline__ void double_round(uint32_t (&x)[16]) {
+  qr_at<FMA, 2 * DR, 0>(x[0], x[4], x[8], x[12]);
+  qr_at<FMA, 2 * DR, 1>(x[1], x[5], x[9], x[13]);
+  qr_at<FMA, 2 * DR, 2>(x[2], x[6], x[10], x[14]);
+  qr_at<FMA, 2 * DR, 3>(x[3], x[7], x[11], x[15]);
+  qr_at<FMA, 2 * DR + 1, 0>(x[0], x[5], x[10], x[15]);
+  qr_at<FMA, 2 * DR + 1, 1>(x[1], x[6], x[11], x[12]);
+  qr_at<FMA, 2 * DR + 1, 2>(x[2], x[7], x[8], x[13]);
+  qr_at<FMA, 2 * DR + 1, 3>(x[3], x[4], x[9], x[14]);
+}
+
+// ChaCha8Prg::expand.  tl/tr are 0 or 1.  FMA balances the two integer pipes
+// (throughput); without it every rotation is one ALU instruction, a shorter
+// dependent chain for code that walks a path with few warps at work.
+template <bool FMA = true>
 __device__ __forceinline__ void prg_expand(const uint4 s, uint4& L, uint4& R, uint32_t& tl,
                                            uint32_t& tr) {
-  uint32_t x0 = kSigma0, x1 = kSigma1, x2 = kSigma2, x3 = kSigma3;
-  uint32_t x4 = s.x, x5 = s.y, x6 = s.z, x7 = s.w;
-  uint32_t x8 = s.x, x9 = s.y, x10 = s.z, x11 = s.w;
-  uint32_t x12 = 0u, x13 = 0u, x14 = 0u, x15 = 0u;
-  uint32_t y0 = kSigma0, y1 = kSigma1, y2 = kSigma2, y3 = kSigma3;
-  uint32_t y4 = s.x, y5 = s.y, y6 = s.z, y7 = s.w;
-  uint32_t y8 = s.x, y9 = s.y, y10 = s.z, y11 = s.w;
-  uint32_t y12 = 1u, y13 = 0u, y14 = 0u, y15 = 0u;
-  MG_DOUBLE_ROUND(x) MG_DOUBLE_ROUND(y)
-  MG_DOUBLE_ROUND(x) MG_DOUBLE_ROUND(y)
-  MG_DOUBLE_ROUND(x) MG_DOUBLE_ROUND(y)
-  MG_DOUBLE_ROUND(x) MG_DOUBLE_ROUND(y)
-  L = make_uint4(x0 + kSigma0, x1 + kSigma1, x2 + kSigma2, x3 + kSigma3);
-  R = make_uint4(x4 + s.x, x5 + s.y, x6 + s.z, x7 + s.w);
-  tl = (y0 + kSigma0) & 1u;
-  tr = (y1 + kSigma1) & 1u;
-  (void)x8; (void)x9; (void)x10; (void)x11; (void)x12; (void)x13; (void)x14; (void)x15;
-  (void)y2; (void)y3; (void)y4; (void)y5; (void)y6; (void)y7; (void)y8; (void)y9;
-  (void)y10; (void)y11; (void)y12; (void)y13; (void)y14; (void)y15;
+  uint32_t x[16] = {kSigma0, kSigma1, kSigma2, kSigma3, s.x, s.y, s.z, s.w, s.x, s.y, s.z, s.w, 0u, 0u, 0u, 0u};
+  uint32_t y[16] = {kSigma0, kSigma1, kSigma2, kSigma3, s.x, s.y, s.z, s.w, s.x, s.y, s.z, s.w, 1u, 0u, 0u, 0u};
+  double_round<FMA, 0>(x); double_round<FMA, 0>(y);
+  double_round<FMA, 1>(x); double_round<FMA, 1>(y);
+  double_round<FMA, 2>(x); double_round<FMA, 2>(y);
+  double_round<FMA, 3>(x); double_round<FMA, 3>(y);
+  L = make_uint4(x[0] + kSigma0, x[1] + kSigma1, x[2] + kSigma2, x[3] + kSigma3);
+  R = make_uint4(x[4] + s.x, x[5] + s.y, x[6] + s.z, x[7] + s.w);
+  tl = (y[0] + kSigma0) & 1u;
+  tr = (y[1] + kSigma1) & 1u;
 }
 
 // One GGM node expansion with the level's correction word applied to both
 // children when t == 1 (dpf.rs:221-239).
+template <bool FMA = true>
 __device__ __forceinline__ void expand_cw(const uint4 s, const uint32_t t, const KeyDev& k,
                                           const uint32_t level, uint4& L, uint32_t& tl, uint4& R,
                                           uint32_t& tr) {
   const uint4 cw = k.cw_seed[level];
   const uint32_t cwl = k.cw_tl[level];
   const uint32_t cwr = k.cw_tr[level];
-  prg_expand(s, L, R, tl, tr);
+  prg_expand<FMA>(s, L, R, tl, tr);
   const uint32_t m = (t == 1u) ? 0xFFFFFFFFu : 0u;
   L.x ^= cw.x & m; L.y ^= cw.y & m; L.z ^= cw.z & m; L.w ^= cw.w & m;
   R.x ^= cw.x & m; R.y ^= cw.y & m; R.z ^= cw.z & m; R.w ^= cw.w & m;
@@ -126,13 +159,14 @@ __device__ __forceinline__ uint4 leaf_mask(const uint4 s, const uint32_t t, cons
 
 // Same as expand_cw with the key read through the read-only data path (the
 // key is uniform across a warp, so every load is a broadcast L1 hit).
+template <bool FMA = true>
 __device__ __forceinline__ void expand_cw_g(const uint4 s, const uint32_t t, const KeyDev* __restrict__ k,
                                             const uint32_t level, uint4& L, uint32_t& tl, uint4& R,
                                             uint32_t& tr) {
   const uint4 cw = __ldg(&k->cw_seed[level]);
   const uint32_t cwl = __ldg(&k->cw_tl[level]);
   const uint32_t cwr = __ldg(&k->cw_tr[level]);
-  prg_expand(s, L, R, tl, tr);
+  prg_expand<FMA>(s, L, R, tl, tr);
   const uint32_t m = (t == 1u) ? 0xFFFFFFFFu : 0u;
   L.x ^= cw.x & m; L.y ^= cw.y & m; L.z ^= cw.z & m; L.w ^= cw.w & m;
   R.x ^= cw.x & m; R.y ^= cw.y & m; R.z ^= cw.z & m; R.w ^= cw.w & m;
@@ -146,33 +180,49 @@ __device__ __forceinline__ uint4 leaf_mask_g(const uint4 s, const uint32_t t, co
   return make_uint4(s.x ^ (f.x & m), s.y ^ (f.y & m), s.z ^ (f.z & m), s.w ^ (f.w & m));
 }
 
-// expand_cw_g with t carried as a mask (KeyAux): m is all ones iff the
-// parent's t == 1; ml / mr are the children's masks.
-__device__ __forceinline__ void expand_cw_m(const uint4 s, const uint32_t m, const KeyDev* __restrict__ k,
-                                            const KeyAux* __restrict__ a, const uint32_t level, uint4& L,
-                                            uint32_t& ml, uint4& R, uint32_t& mr) {
+// The level's correction word on a node's children as prg_expand gives them
+// (seeds L, R, bits bl, br), with t carried as a mask (KeyAux): m is all ones
+// iff the parent's t == 1; ml / mr are the children's masks.
+__device__ __forceinline__ void apply_cw_m(uint4& L, uint4& R, const uint32_t bl, const uint32_t br, const uint32_t m,
+                                           const KeyDev* __restrict__ k, const KeyAux* __restrict__ a,
+                                           const uint32_t level, uint32_t& ml, uint32_t& mr) {
   const uint4 cw = __ldg(&k->cw_seed[level]);
   const uint4 tm = __ldg(&a->cw_tm[level]);
-  uint32_t tl, tr;
-  prg_expand(s, L, R, tl, tr);
   L.x ^= cw.x & m; L.y ^= cw.y & m; L.z ^= cw.z & m; L.w ^= cw.w & m;
   R.x ^= cw.x & m; R.y ^= cw.y & m; R.z ^= cw.z & m; R.w ^= cw.w & m;
-  ml = ((0u - tl) ^ (tm.x & m)) & ~(tm.y & m);
-  mr = ((0u - tr) ^ (tm.z & m)) & ~(tm.w & m);
+  ml = ((0u - bl) ^ (tm.x & m)) & ~(tm.y & m);
+  mr = ((0u - br) ^ (tm.z & m)) & ~(tm.w & m);
 }
 
 // Last level (level d - 1): both children's leaf masks straight from the PRG
 // seeds, with the level's correction word and the final correction word
 // folded into one table entry per child.
-__device__ __forceinline__ void leaf_pair_m(const uint4 s, const uint32_t m, const KeyAux* __restrict__ a,
-                                            uint4& mask_l, uint4& mask_r) {
-  uint32_t bl, br;
-  prg_expand(s, mask_l, mask_r, bl, br);
+__device__ __forceinline__ void leaf_terms_m(const uint4 L, const uint4 R, const uint32_t bl, const uint32_t br,
+                                             const uint32_t m, const KeyAux* __restrict__ a, uint4& mask_l,
+                                             uint4& mask_r) {
   const uint32_t p2 = m & 2u;  // 2 * parent bit
   const uint4 cl = __ldg(&a->leaf[p2 | bl]);
   const uint4 cr = __ldg(&a->leaf[4u + (p2 | br)]);
-  mask_l.x ^= cl.x; mask_l.y ^= cl.y; mask_l.z ^= cl.z; mask_l.w ^= cl.w;
-  mask_r.x ^= cr.x; mask_r.y ^= cr.y; mask_r.z ^= cr.z; mask_r.w ^= cr.w;
+  mask_l = make_uint4(L.x ^ cl.x, L.y ^ cl.y, L.z ^ cl.z, L.w ^ cl.w);
+  mask_r = make_uint4(R.x ^ cr.x, R.y ^ cr.y, R.z ^ cr.z, R.w ^ cr.w);
+}
+
+// One node expansion with the level's correction word, t carried as a mask.
+__device__ __forceinline__ void expand_cw_m(const uint4 s, const uint32_t m, const KeyDev* __restrict__ k,
+                                            const KeyAux* __restrict__ a, const uint32_t level, uint4& L,
+                                            uint32_t& ml, uint4& R, uint32_t& mr) {
+  uint32_t bl, br;
+  prg_expand(s, L, R, bl, br);
+  apply_cw_m(L, R, bl, br, m, k, a, level, ml, mr);
+}
+
+// The leaf pair below node s of level d - 1.
+__device__ __forceinline__ void leaf_pair_m(const uint4 s, const uint32_t m, const KeyAux* __restrict__ a,
+                                            uint4& mask_l, uint4& mask_r) {
+  uint4 L, R;
+  uint32_t bl, br;
+  prg_expand(s, L, R, bl, br);
+  leaf_terms_m(L, R, bl, br, m, a, mask_l, mask_r);
 }
 
 __device__ __forceinline__ uint4 xor_and(uint4 acc, const uint4 d, const uint4 m) {
@@ -221,11 +271,20 @@ struct ScanParams {
 // item is 32 consecutive frontier nodes of one key group ("warp tile", 32 x
 // 2^M rows); each lane walks its node's 2^M leaves depth-first.
 
-// Widest CTA of the warp-independent kernel (16 warps, one CTA per SM: the
-// 128 registers per thread of 512 threads fill the register file); CTAs of
-// 8 or 4 warps are used when 16 warps' stacks do not fit.
-constexpr int kWarpThreads = 512;
-constexpr int kWarps = kWarpThreads / 32;
+// Rows of at most 32 B with one key per warp: every lane scans its own
+// subtree's rows (the own-rows scan); wider rows or several keys exchange the
+// leaf masks through shared memory.
+__host__ __device__ constexpr bool own_rows(int G, uint32_t VT) { return G == 1 && VT <= 2; }
+
+// Widest CTA of the warp-independent kernel, one CTA per SM: 16 warps (128
+// registers a thread), or 20 (102) for the own-rows scan, whose registers fit
+// 96.  With the ALU and FMA pipes both near their limit a fifth warp per
+// scheduler hides what is left of the fixed-latency waits: 2^28 x 32 B with
+// 3 keys 19.8-20.0 ms against 20.1-20.3 with 16.  Half or a quarter as many
+// when the stacks do not fit the shared memory.
+constexpr int kWarps = 16;
+constexpr int kOwnWarps = 20;
+__host__ __device__ constexpr int warp_cta_warps(int G, uint32_t VT) { return own_rows(G, VT) ? kOwnWarps : kWarps; }
 
 struct WarpSeg {
   const uint4* table;   // rows * V uint4

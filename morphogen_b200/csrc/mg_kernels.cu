@@ -76,7 +76,7 @@ __global__ void __launch_bounds__(kThreads, (G <= 4 ? 3 : 2)) scan_kernel(const 
       for (uint32_t lvl = 0; lvl < L0; ++lvl) {
         uint4 Lc, Rc;
         uint32_t tl, tr;
-        expand_cw(s, t, K, lvl, Lc, tl, Rc, tr);
+        expand_cw<false>(s, t, K, lvl, Lc, tl, Rc, tr);
         const uint32_t bit = (tile >> (L0 - 1 - lvl)) & 1u;
         s = bit ? Rc : Lc;
         t = bit ? tr : tl;
@@ -286,7 +286,7 @@ __global__ void __launch_bounds__(kThreads) frontier_kernel(const __grid_constan
       for (uint32_t lvl = 0; lvl < f.L_in; ++lvl) {
         uint4 Lc, Rc;
         uint32_t tl, tr;
-        expand_cw_g(s, t, K, lvl, Lc, tl, Rc, tr);
+        expand_cw_g<false>(s, t, K, lvl, Lc, tl, Rc, tr);
         const uint32_t bit = (uint32_t)(a >> (f.L_in - 1 - lvl)) & 1u;
         s = bit ? Rc : Lc;
         t = bit ? tr : tl;
@@ -353,8 +353,12 @@ __device__ __forceinline__ void xor_out(uint4* out, const uint4 v) {
 // one leaf pair per lane for every key.  Accumulators stay in registers and
 // are flushed (warp shuffle XOR) into the warp's own partial row when the
 // group or segment changes.
-// For rows of VT * G <= 2 uint4 each lane ANDs its own two rows with its own
-// masks.  Otherwise the masks are exchanged through shared memory with
+// For rows of at most 32 B with one key per warp each lane ANDs its own two
+// rows with its own masks; the walk holds two copies of the PRG code, one for
+// internal nodes and one for leaf pairs (about 25 KB, where a third copy runs
+// into the instruction cache: 2^25 x 32 B, 3 keys 2.80 ms with three copies,
+// 2.65 with one and a stack round trip per step, 2.61 with two; 2.56 with 20
+// warps).  Otherwise the masks are exchanged through shared memory with
 // __syncwarp only, and the warp scans the step's 64 rows (32 runs of 2) with
 // coalesced 128-bit loads; VT divides 32, so a lane always holds the same
 // 16-byte position of a row.  The first 8 of a lane's loads of a step are
@@ -388,42 +392,19 @@ __device__ __forceinline__ void leaf_walk(const KeyDev* __restrict__ K, const Ke
   leaf_pair_m(s, m, A, ml, mr);
 }
 
-// Two depth-first steps at once (M >= 2): node q of relative level M - 2,
-// whose children are the nodes of leaf pairs 2q and 2q + 1.  The path
-// re-joins the stack at relative level M - 1 - ffs(q) (the root for q == 0),
-// pushes the right children it passes and expands node q itself, so the
-// second child stays in registers instead of taking a stack round trip.
-__device__ __forceinline__ void pair_walk(const KeyDev* __restrict__ K, const KeyAux* __restrict__ A,
-                                          uint4* col_seed, int8_t* col_t, uint32_t q, uint32_t M, uint32_t F,
-                                          uint4& s0, uint32_t& m0, uint4& s1, uint32_t& m1) {
-  uint32_t lvl = q ? (M - 1 - (uint32_t)__ffs((int)q)) : 0u;
-  uint4 s = col_seed[lvl * 32];
-  uint32_t m = (uint32_t)(int32_t)col_t[lvl * 32];
-  for (; lvl < M - 2; ++lvl) {
-    uint4 Lc, Rc;
-    uint32_t mlc, mrc;
-    expand_cw_m(s, m, K, A, F + lvl, Lc, mlc, Rc, mrc);
-    col_seed[(lvl + 1) * 32] = Rc;
-    col_t[(lvl + 1) * 32] = (int8_t)mrc;
-    s = Lc;
-    m = mlc;
-  }
-  expand_cw_m(s, m, K, A, F + M - 2, s0, m0, s1, m1);
-}
-
 template <int G, int VT>
-__global__ void __launch_bounds__(kWarpThreads, 1) scan_warp_kernel(const __grid_constant__ WarpScanParams p) {
+__global__ void __launch_bounds__(warp_cta_warps(G, VT) * 32, 1) scan_warp_kernel(const __grid_constant__ WarpScanParams p) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ uint32_t s_next;  // next item of this CTA's range
   constexpr int NL = 2 * VT;            // uint4 loads per lane per step
   constexpr int PF = NL < MG_WARP_PREFETCH ? NL : MG_WARP_PREFETCH;  // loads issued before the ChaCha work
   constexpr uint32_t RPL = 32 / VT;     // rows covered by one warp-wide load
-  // Rows of at most 32 B (one key per warp) or 16 B (two): every lane scans
+  // Rows of at most 32 B with one key per warp: every lane scans
   // its own subtree's two rows of the step (64 contiguous bytes, whole
   // sectors) against its own leaf masks, with no shared-memory exchange and
   // VT accumulators per key.  Wider rows use the exchange, which keeps the
   // loads coalesced and the register count flat.
-  constexpr bool OWN = VT * G <= 2;
+  constexpr bool OWN = own_rows(G, VT);
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   const uint32_t nw = blockDim.x >> 5;
   const uint32_t slots = p.slots;
@@ -545,60 +526,47 @@ __global__ void __launch_bounds__(kWarpThreads, 1) scan_warp_kernel(const __grid
     const uint4* const own_lp = full ? tbl + (row0 + ((uint64_t)lane << M)) * VT : tbl;
     auto run_own = [&](auto full_tag) {
     constexpr bool FULL = decltype(full_tag)::value;
-    if constexpr (FULL && G == 1) {
-      // Odd leaf pairs are the right children of the even steps' last
-      // expansion: they stay in registers (carry) instead of taking a
-      // stack round trip.
-      if (M >= 2) {
-        const KeyDev* __restrict__ K0 = kp;
-        const KeyAux* __restrict__ A0 = ap;
-        uint4 carry_s = make_uint4(0u, 0u, 0u, 0u);
-        uint32_t carry_m = 0u;
-        for (uint32_t pi = 0; pi < pairs; ++pi) {
-          uint4 dat[2 * AV];
+    for (uint32_t pi = 0; pi < pairs; pi += 2) {
+      // Walk to the node of leaf pair pi and, when M >= 2, its sibling, the
+      // node of pair pi + 1: the path re-joins the stack at relative level
+      // M - ffs(pi) (the root for pi == 0) and pushes the right children it
+      // passes, the last one staying in registers.
+      uint32_t lvl = pi ? (M - (uint32_t)__ffs((int)pi)) : 0u;
+      uint4 s0 = w_seed[lvl * 32 + lane], s1 = make_uint4(0u, 0u, 0u, 0u);
+      uint32_t m0 = (uint32_t)(int32_t)w_t[lvl * 32 + lane], m1 = 0u;
+#pragma unroll 1
+      for (; lvl + 1 < M; ++lvl) {
+        uint32_t mlc;
+        uint4 Lc;
+        expand_cw_m(s0, m0, kp, ap, F + lvl, Lc, mlc, s1, m1);
+        if (lvl + 2 < M) {
+          w_seed[(lvl + 1) * 32 + lane] = s1;
+          w_t[(lvl + 1) * 32 + lane] = (int8_t)m1;
+        }
+        s0 = Lc;
+        m0 = mlc;
+      }
+#pragma unroll 1
+      for (uint32_t h = 0; h < 2u && pi + h < pairs; ++h) {
+        uint4 dat[2 * AV];
 #pragma unroll
-          for (int j = 0; j < 2 * AV; ++j) dat[j] = __ldg(own_lp + (size_t)pi * (2 * VT) + j);
-          uint4 sl;
-          uint32_t msl;
-          if (pi & 1u) {
-            sl = carry_s;
-            msl = carry_m;
+        for (int j = 0; j < 2 * AV; ++j) {
+          if constexpr (FULL) {
+            dat[j] = __ldg(own_lp + (size_t)(pi + h) * (2 * VT) + j);
           } else {
-            pair_walk(K0, A0, w_seed + lane, w_t + lane, pi >> 1, M, F, sl, msl, carry_s, carry_m);
-          }
-          uint4 ml, mr;
-          leaf_pair_m(sl, msl, A0, ml, mr);
-#pragma unroll
-          for (int v = 0; v < AV; ++v) {
-            own[0][v] = xor_and(own[0][v], dat[v], ml);
-            own[0][v] = xor_and(own[0][v], dat[AV + v], mr);
+            const uint64_t row = row0 + ((uint64_t)lane << M) + 2u * (pi + h) + (uint32_t)(j / AV);
+            dat[j] = row < nrows ? __ldg(tbl + row * VT + (j % AV)) : make_uint4(0u, 0u, 0u, 0u);
           }
         }
-        return;
-      }
-    }
-    for (uint32_t pi = 0; pi < pairs; ++pi) {
-      uint4 dat[2 * AV];
-#pragma unroll
-      for (int j = 0; j < 2 * AV; ++j) {
-        if constexpr (FULL) {
-          dat[j] = __ldg(own_lp + (size_t)pi * (2 * VT) + j);
-        } else {
-          const uint64_t row = row0 + ((uint64_t)lane << M) + 2u * pi + (uint32_t)(j / AV);
-          dat[j] = row < nrows ? __ldg(tbl + row * VT + (j % AV)) : make_uint4(0u, 0u, 0u, 0u);
-        }
-      }
-#pragma unroll
-      for (int k = 0; k < G; ++k) {
-        if ((uint32_t)k >= g) break;
         uint4 ml, mr;
-        leaf_walk(kp + k, ap + k, w_seed + (size_t)k * slots * 32 + lane, w_t + (size_t)k * slots * 32 + lane,
-                  pi, M, F, ml, mr);
+        leaf_pair_m(s0, m0, ap, ml, mr);
 #pragma unroll
         for (int v = 0; v < AV; ++v) {
-          own[k][v] = xor_and(own[k][v], dat[v], ml);
-          own[k][v] = xor_and(own[k][v], dat[AV + v], mr);
+          own[0][v] = xor_and(own[0][v], dat[v], ml);
+          own[0][v] = xor_and(own[0][v], dat[AV + v], mr);
         }
+        s0 = s1;
+        m0 = m1;
       }
     }
     };
@@ -719,7 +687,7 @@ __global__ void __launch_bounds__(kWarpThreads, 1) scan_warp_kernel(const __grid
 
 // Whether scan_warp_kernel<G, VT> reduces its partial rows into the shares
 // itself (wide rows) or leaves them to reduce_kernel (own-rows scan).
-bool warp_reduces_in_kernel(int G, uint32_t VT) { return (uint32_t)G * VT > 2u; }
+bool warp_reduces_in_kernel(int G, uint32_t VT) { return !own_rows(G, VT); }
 
 // out[c] ^= XOR over the nparts partial rows (launch_reduce zeroes out first).
 // Block (x, y) = cpb columns x (kThreads / cpb) slices over the partial rows
