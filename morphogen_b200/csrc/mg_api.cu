@@ -360,12 +360,14 @@ struct SegPlan {
   bool warp;
 };
 
-// Keys evaluated together on one work item.  Rows of up to 128 B leave the
-// pass bound by ChaCha8 issue slots, so one key per item maximises the
-// number of independent items (re-reads of a row by sibling items hit L2);
-// wider rows share each row load across up to 4 keys.
+// Keys evaluated together on one work item.  Warp kernel: one key for rows of
+// up to 64 B, whose lanes hold a pair's rows in registers beside the ChaCha
+// state; three (a query's keys) share each row load and its address work for
+// wider ones (3 keys, 2^22 x 128 B: 414 us against 437 with one; 10^6 x 96 B:
+// 125 against 132; equal at 48 B).  CTA kernel: one key up to 128 B, where the
+// pass is bound by ChaCha8 issue slots, else up to 4.
 int choose_g(uint32_t V, size_t nkeys, uint32_t pinned, bool warp) {
-  int g = pinned ? (int)pinned : (V <= 8 ? 1 : 4);
+  int g = pinned ? (int)pinned : warp ? (V <= 4 ? 1 : 3) : (V <= 8 ? 1 : 4);
   if (warp && g > 4) g = 4;
   if ((size_t)g > nkeys) g = (int)nkeys;
   if (g < 1) g = 1;
@@ -852,56 +854,79 @@ int plan_cta(mg_batch* b, const std::vector<SegPlan>& segs, int G, uint32_t col0
   }
 }
 
+// Expected microseconds of a warp-kernel launch that depend on its depth M:
+// the frontier, and the schedulers' rounds of items.  An item is G keys' 2^M - 1
+// node expansions of a warp and V * 2^M row loads per lane; with w of its W
+// warps at work a scheduler runs at the fraction kRate[w] of its full rate.
+// The constants are fitted to passes timed at every M from 1 to 10 (21
+// workloads of 4099 rows to 2^25, 32 to 512 B, 1 to 48 keys): the M it picks is
+// within 3.5% of the fastest in all of them, where the deepest M whose items
+// round up by at most 3% over the schedulers, the rule before, lost up to 54%
+// (300000 x 192 B, 12 keys: 221 us against 144; 100000 x 64 B: 37 against 33).
+double warp_cost_us(uint64_t items, double item_nodes, double item_loads, uint64_t frontier_nodes, int G, bool regroups,
+                    uint32_t nw, int sms) {
+  constexpr double kNode = 0.435;         // a warp's node expansion on a busy scheduler
+  constexpr double kLoad = 0.0051;        // a warp-wide row load, and
+  constexpr double kLoadKey = 0.0078;     // its AND/XOR per key
+  constexpr double kItem = 0.22;          // taking an item
+  constexpr double kRegroup = 2.0;        // and changing to another key group's accumulators
+  constexpr double kFrontier = 0.037e-3;  // a frontier node
+  constexpr double kTail = 0.11;          // of an item per warp: warps drift, the last rows are waited for
+  constexpr double kRate[5] = {0.62, 0.72, 0.82, 0.96, 1.0};
+  const uint64_t W = std::max<uint64_t>(1, nw / 4);
+  const uint64_t q = (items + (uint64_t)sms * 4 - 1) / ((uint64_t)sms * 4);
+  const double item = kNode * item_nodes + item_loads * (kLoad + kLoadKey * G) + kItem + (regroups ? kRegroup : 0.0);
+  const double rounds = (double)(q / W) * (double)W / kRate[W - 1] + (q % W ? (double)(q % W) / kRate[q % W - 1] : 0.0);
+  return kFrontier * (double)frontier_nodes + item * (rounds + kTail * (double)std::min(W, q));
+}
+
 // Plan one warp-kernel launch over segs (same V, at most kMaxSegs): depth-first
-// levels per lane M and the CTA width (16 warps, one CTA per SM, when their
-// stacks fit the shared memory, else 8 or 4 warps).  The CTAs take their items
-// dynamically, so an SM's four schedulers finish within about one item of one
-// another; M is the deepest whose items per scheduler round up by at most 3%
-// (fewer, deeper items need fewer frontier nodes), or pinned as
-// subtree_bits = M + 5.
+// levels per lane M (the cheapest by warp_cost_us, or pinned as subtree_bits =
+// M + 5) and the CTA width.
 int plan_warp(mg_batch* b, const std::vector<SegPlan>& segs, int G, uint32_t VT, uint32_t col0,
               size_t& key_cursor, std::vector<uint32_t>& key_col, std::vector<uint32_t>& key_bytes,
               std::vector<uint32_t>& key_slot, uint64_t& fr_cursor, size_t& tmp_need, mg_batch::Launch& out) {
   mg_context* ctx = b->ctx;
-  struct Cand { uint32_t M; double bal; uint64_t items; int occ; size_t smem; uint32_t nw; };
+  struct Shape { uint32_t slots, nw; size_t smem; };
+  struct Cand { uint32_t M; double cost; Shape sh; };
+  // The widest CTA whose shared memory fits.
+  auto shape_of = [&](uint32_t M, Shape& sh) {
+    sh.slots = mg::warp_slots(G, VT, M);
+    for (sh.nw = (uint32_t)mg::warp_cta_warps(G); sh.nw >= 4; sh.nw -= 4) {
+      sh.smem = mg::warp_smem_bytes(G, VT, sh.slots, sh.nw);
+      if (sh.smem <= ctx->smem_optin) return true;
+    }
+    return false;
+  };
   std::vector<Cand> cands;
   const uint32_t pinned = b->eff_S;
   for (uint32_t Mt = 10; Mt >= 1; --Mt) {
     if (pinned && !(pinned >= 6 ? Mt == pinned - 5 : Mt == 1)) continue;
-    uint64_t items = 0;
-    uint32_t slots = 1;
+    uint64_t items = 0, nodes = 0;
+    double item_nodes = 0, item_loads = 0;
+    bool regroups = segs.size() > 1;
+    uint32_t Mmax = 1;
     for (const SegPlan& sp : segs) {
       const uint32_t M = std::min(Mt, sp.d);
       const uint64_t nF = level_count(sp.table, M);
-      items += (sp.keys.size() / sp.g) * ((nF + 31) / 32);
-      slots = std::max(slots, M);
+      const uint64_t groups = sp.keys.size() / sp.g, n = groups * ((nF + 31) / 32);
+      items += n;
+      nodes += sp.keys.size() * nF;
+      item_nodes += (double)n * sp.g * ((1u << M) - 1u);
+      item_loads += (double)n * VT * (1u << M);
+      regroups = regroups || groups > 1;
+      Mmax = std::max(Mmax, M);
     }
-    uint32_t nw = mg::warp_cta_warps(G, VT);
-    size_t smem = mg::warp_smem_bytes(G, VT, slots, nw);
-    while (smem > ctx->smem_optin && nw > 4) {
-      nw /= 2;
-      smem = mg::warp_smem_bytes(G, VT, slots, nw);
-    }
-    if (smem > ctx->smem_optin) continue;
-    if (int rc = prepare_warp(ctx, G, VT, smem)) return rc;
-    const int occ = mg::warp_occupancy(G, VT, smem, nw);
-    if (occ <= 0) continue;
-    // Items per warp scheduler (4 per SM), rounded up: the last item of
-    // the busiest scheduler bounds the pass.
-    const uint64_t sched = (uint64_t)ctx->sms * 4;
-    const uint64_t worst = (items + sched - 1) / sched;
-    const double bal = worst ? (double)items / ((double)worst * (double)sched) : 1.0;
-    cands.push_back({Mt, bal, items, occ, smem, nw});
+    Shape sh;
+    if (!shape_of(Mmax, sh)) continue;
+    const double n = std::max<double>(1.0, (double)items);
+    cands.push_back({Mt, warp_cost_us(items, item_nodes / n, item_loads / n, nodes, G, regroups && G > 1, sh.nw, ctx->sms),
+                     sh});
   }
   if (cands.empty()) return fail(MG_EINVAL, "no warp-kernel shape fits the device (G=%d)", G);
-  const Cand* best = nullptr;
+  const Cand* best = &cands[0];
   for (const Cand& c : cands)
-    if (c.bal >= 0.97) { best = &c; break; }  // deepest balanced
-  if (!best) {
-    best = &cands[0];
-    for (const Cand& c : cands)
-      if (c.bal > best->bal + 0.01) best = &c;
-  }
+    if (c.cost < best->cost) best = &c;
 
   mg_batch::Launch L;
   std::memset(&L.w, 0, sizeof L.w);
@@ -910,7 +935,7 @@ int plan_warp(mg_batch* b, const std::vector<SegPlan>& segs, int G, uint32_t VT,
   L.VT = VT;
   L.col0 = col0;
   uint64_t items = 0;
-  uint32_t cols = 0, slots = 1;
+  uint32_t cols = 0;
   size_t cursor = key_cursor;
   for (size_t si = 0; si < segs.size(); ++si) {
     const SegPlan& sp = segs[si];
@@ -972,30 +997,27 @@ int plan_warp(mg_batch* b, const std::vector<SegPlan>& segs, int G, uint32_t VT,
     cursor += nk;
     items += (uint64_t)sg.groups * sg.tiles;
     cols += nk * VT;
-    slots = std::max(slots, M);
   }
   L.w.nsegs = (uint32_t)segs.size();
   L.w.items = items;
   L.w.cols = cols;
-  L.w.slots = slots;
+  L.w.V = VT;
+  L.w.slots = best->sh.slots;
   L.cols = cols;
-  L.NW = best->nw;
-  // A CTA's warps take its items in rounds.  When a CTA holds only a few
-  // rounds and 16 warps leave much of the last one idle (4096 items on 148
-  // CTAs: 27.7 per CTA, 1.73 per warp), 14 warps fill it (1.98 per warp):
-  // measured 1% faster on the 2^20 x 256 B pass.  With many rounds the
-  // 16 warps' latency hiding counts for more.
-  if (L.NW == (uint32_t)mg::kWarps) {
-    const double ipc = (double)items / (double)ctx->sms;
-    auto fill = [&](uint32_t w) { return ipc / ((double)w * std::ceil(ipc / (double)w)); };
-    if (std::ceil(ipc / mg::kWarps) <= 4.0 && fill(14) > fill(mg::kWarps) + 0.05 &&
-        mg::warp_smem_bytes(G, VT, slots, 14) <= ctx->smem_optin)
-      L.NW = 14;
-  }
+  L.NW = best->sh.nw;
+  auto smem_at = [&](uint32_t nw) {
+    return mg::warp_smem_bytes(G, VT, L.w.slots, nw);
+  };
   // Fewer items than the device has warps: CTAs just wide enough to spread
   // them over all SMs, so that no scheduler holds two while another has none.
   L.NW = (uint32_t)std::min<uint64_t>(L.NW, std::max<uint64_t>(1, (items + ctx->sms - 1) / ctx->sms));
-  L.smem = mg::warp_smem_bytes(G, VT, slots, L.NW);
+  L.smem = smem_at(L.NW);
+  // With few items per warp, four queues per CTA: one would let the last items
+  // fall to warps of the same scheduler while another runs dry (28 items of a
+  // 2^20 x 256 B pass on 16 warps then take 8 item times of a scheduler
+  // instead of 7: 145 us against 137).  With many, one queue evens out the
+  // warps' drift (2^25 x 32 B: 2.54 ms against 2.57).
+  L.w.queues = items <= (uint64_t)4 * L.NW * ctx->sms ? 4u : 1u;
   if (int rc = prepare_warp(ctx, G, VT, L.smem)) return rc;
   const int occ = mg::warp_occupancy(G, VT, L.smem, L.NW);
   if (occ <= 0) return fail(MG_EINVAL, "warp kernel does not fit the device");
@@ -1068,27 +1090,36 @@ int plan_pass(mg_batch* b) {
     it->keys.push_back(i);
   }
 
-  // Kernel per segment: the warp kernel for rows of 16..512 B (V dividing
-  // 32) and d >= 1, the CTA kernel otherwise.
+  // Kernel per segment: the warp kernel for rows of 16..512 B and d >= 1, the
+  // CTA kernel otherwise.  A caller may pin the warp kernel for row sizes that
+  // are powers of two only.
   for (SegPlan& sp : segs) {
     const uint32_t V = sp.table->row_bytes / 16;
     const bool ok = mg::warp_vt_supported(V) && sp.d >= 1;
-    if (b->eff_kind == MG_KERNEL_WARP && !ok)
+    if (b->eff_kind == MG_KERNEL_WARP && (!ok || (b->kind_pref == MG_KERNEL_WARP && (V & (V - 1)) != 0)))
       return fail(MG_EINVAL, "the warp kernel needs row_bytes in {16..512, powers of two} and d >= 1");
     sp.warp = ok && b->eff_kind != MG_KERNEL_CTA;
   }
-  uint32_t Vc = 1, Vw = 1;
-  size_t nc = 1, nwk = 1;
+  // Keys per item: one choice for the CTA kernel, one per row size for the
+  // warp kernel (each row size is a launch of its own).
+  uint32_t Vc = 1;
+  size_t nc = 1;
+  std::map<uint32_t, size_t> warp_keys;  // V -> most keys of a segment
   for (const SegPlan& sp : segs) {
     const uint32_t V = sp.table->row_bytes / 16;
-    if (sp.warp) { Vw = std::max(Vw, V); nwk = std::max(nwk, sp.keys.size()); }
-    else { Vc = std::max(Vc, V); nc = std::max(nc, sp.keys.size()); }
+    if (sp.warp) {
+      warp_keys[V] = std::max(warp_keys[V], sp.keys.size());
+    } else {
+      Vc = std::max(Vc, V);
+      nc = std::max(nc, sp.keys.size());
+    }
   }
   const int Gc = choose_g(Vc, nc, b->eff_G, false);
-  const int Gw = choose_g(Vw, nwk, b->eff_G, true);
+  std::map<uint32_t, int> Gw;
+  for (const auto& vk : warp_keys) Gw[vk.first] = choose_g(vk.first, vk.second, b->eff_G, true);
   std::vector<SegPlan> split;
   for (SegPlan& sp : segs) {
-    const int G = sp.warp ? Gw : Gc;
+    const int G = sp.warp ? Gw[sp.table->row_bytes / 16] : Gc;
     const uint32_t g = (uint32_t)std::min<size_t>((size_t)G, sp.keys.size());
     const size_t full = sp.keys.size() / g * g;
     split.push_back(SegPlan{sp.table, sp.d, std::vector<uint32_t>(sp.keys.begin(), sp.keys.begin() + full), g, sp.warp});
@@ -1115,14 +1146,15 @@ int plan_pass(mg_batch* b) {
     total_cols += L.cols;
     launches.push_back(std::move(L));
   }
-  for (uint32_t VT = 1; VT <= 32; VT *= 2) {
+  for (const auto& vg : Gw) {
+    const uint32_t VT = vg.first;
     std::vector<SegPlan> ws;
     for (const SegPlan& sp : split)
       if (sp.warp && sp.table->row_bytes / 16 == VT) ws.push_back(sp);
     for (size_t s0 = 0; s0 < ws.size(); s0 += mg::kMaxSegs) {
       std::vector<SegPlan> chunk(ws.begin() + s0, ws.begin() + std::min(ws.size(), s0 + mg::kMaxSegs));
       mg_batch::Launch L;
-      if (int rc = plan_warp(b, chunk, Gw, VT, total_cols, key_cursor, key_col, key_bytes, key_slot, fr_cursor,
+      if (int rc = plan_warp(b, chunk, vg.second, VT, total_cols, key_cursor, key_col, key_bytes, key_slot, fr_cursor,
                              tmp_need, L))
         return rc;
       total_cols += L.cols;

@@ -12,7 +12,7 @@
 // expansion written with one instruction per operation keeps the ALU pipe full
 // (456 instructions) and the FMA pipe half idle (227).  Rotations by 16 and 8
 // are whole bytes, and a byte-wise dot product plus a multiply-add does one on
-// the FMA pipe (rotl_bytes): with 69 of them there, 387 ALU and 366 FMA
+// the FMA pipe (rotl_bytes): with 70 of them there, about 387 ALU and 366 FMA
 // instructions, 40.2 -> 44.6 G node expansions/s for the PRG alone
 // (mg_prg_peak).  More of them loses to the issue rate (one instruction per
 // clock and scheduler, 755 per expansion), fewer to the ALU pipe.  Both blocks
@@ -96,11 +96,13 @@ __device__ __forceinline__ void quarter_round(uint32_t& a, uint32_t& b, uint32_t
 }
 
 // Which of a block's rotations by 16 and 8 run on the FMA pipe (FMA set), by
-// round and quarter round: the 16s of quarter rounds 1..3 and the 8s of the
-// diagonal rounds, 69 of the 114 that matter.
+// round and quarter round: the 16s of quarter rounds 0..2 and the 8s of the
+// diagonal rounds, about 70 of the 114 that matter.  Which ones matters little
+// for the PRG alone; of 72 such choices this was the best over the pair scan's
+// three kernels (between 2.51 and 2.63 ms for 3 keys over 2^25 x 32 B).
 template <bool FMA, int RD, int C>
 __device__ __forceinline__ void qr_at(uint32_t& a, uint32_t& b, uint32_t& c, uint32_t& d) {
-  quarter_round<FMA && C != 0, FMA && (RD & 1) != 0>(a, b, c, d);
+  quarter_round<FMA && C != 3, FMA && (RD & 1) != 0>(a, b, c, d);
 }
 
 template <bool FMA, int DR>
@@ -271,20 +273,25 @@ struct ScanParams {
 // item is 32 consecutive frontier nodes of one key group ("warp tile", 32 x
 // 2^M rows); each lane walks its node's 2^M leaves depth-first.
 
-// Rows of at most 32 B with one key per warp: every lane scans its own
-// subtree's rows (the own-rows scan); wider rows or several keys exchange the
-// leaf masks through shared memory.
-__host__ __device__ constexpr bool own_rows(int G, uint32_t VT) { return G == 1 && VT <= 2; }
+// One key per warp and rows of 16, 32 or 64 B: the pair scan (a step is one
+// leaf pair per lane, its rows in registers beside the ChaCha state).  Other
+// row sizes up to 512 B, or several keys per warp: the block scan.
+__host__ __device__ constexpr bool pair_scan(int G, uint32_t V) { return G == 1 && (V == 1 || V == 2 || V == 4); }
 
-// Widest CTA of the warp-independent kernel, one CTA per SM: 16 warps (128
-// registers a thread), or 20 (102) for the own-rows scan, whose registers fit
-// 96.  With the ALU and FMA pipes both near their limit a fifth warp per
-// scheduler hides what is left of the fixed-latency waits: 2^28 x 32 B with
-// 3 keys 19.8-20.0 ms against 20.1-20.3 with 16.  Half or a quarter as many
-// when the stacks do not fit the shared memory.
-constexpr int kWarps = 16;
-constexpr int kOwnWarps = 20;
-__host__ __device__ constexpr int warp_cta_warps(int G, uint32_t VT) { return own_rows(G, VT) ? kOwnWarps : kWarps; }
+// Widest CTA of the warp-independent kernels, one CTA per SM; four warps fewer
+// at a time when the shared memory does not hold it.  One key per warp: 20
+// warps, whose registers fit 96.  With the ALU and FMA pipes both near their
+// limit a fifth warp per scheduler hides what is left of the fixed-latency
+// waits (3 keys, 2^28 x 32 B: 19.8-20.0 ms against 20.1-20.3 with 16; 12 keys,
+// 3000000 x 64 B: 0.99 against 1.02).  Several keys: 16 warps, 128 registers.
+__host__ __device__ constexpr int warp_cta_warps(int G) { return G == 1 ? 20 : 16; }
+
+// Leaves per lane of a step (one pair).
+constexpr uint32_t kBlockLeaves = 2;
+
+// Loads per lane and chunk of the block scan's rows.  8 (with 3 keys a 256-B
+// row pair's 32 loads pass in 4 of its 5-6 node expansions); 512-B rows take 16.
+__host__ __device__ constexpr int block_chunk(uint32_t V) { return V == 32 ? 16 : 8; }
 
 struct WarpSeg {
   const uint4* table;   // rows * V uint4
@@ -314,7 +321,9 @@ struct WarpScanParams {
   uint64_t items;
   uint32_t nsegs;
   uint32_t cols;
-  uint32_t slots;       // depth-first stack slots per key per lane (>= max M)
+  uint32_t V;           // uint4 per row of every segment of the launch
+  uint32_t slots;       // stack levels per lane and key
+  uint32_t queues;      // item queues per CTA: 1, or 4 (one per warp scheduler)
 };
 
 // Levels one frontier-chain step expands (its last level's 2^10 nodes fit the

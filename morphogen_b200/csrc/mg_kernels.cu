@@ -342,152 +342,167 @@ __device__ __forceinline__ void xor_out(uint4* out, const uint4 v) {
   atomicXor(o + 1, ((unsigned long long)v.w << 32) | v.z);
 }
 
-// Warp-independent fused expansion + scan.  A CTA of W warps (16 when its
-// shared memory fits, else 8 or 4) owns a contiguous range
-// of the pass's work items, in (tile, key group) order with the groups of a
-// tile next to each other; its warps take the items one at a time from a
-// shared-memory counter, so warps that share an SMSP with fewer busy warps
-// simply take more items and every SM finishes within about one item of the
-// others.  Per item each lane loads its frontier node and walks its 2^M
-// leaves depth-first (stack in the warp's shared-memory slice); a step yields
-// one leaf pair per lane for every key.  Accumulators stay in registers and
-// are flushed (warp shuffle XOR) into the warp's own partial row when the
-// group or segment changes.
-// For rows of at most 32 B with one key per warp each lane ANDs its own two
-// rows with its own masks; the walk holds two copies of the PRG code, one for
-// internal nodes and one for leaf pairs (about 25 KB, where a third copy runs
-// into the instruction cache: 2^25 x 32 B, 3 keys 2.80 ms with three copies,
-// 2.65 with one and a stack round trip per step, 2.61 with two; 2.56 with 20
-// warps).  Otherwise the masks are exchanged through shared memory with
-// __syncwarp only, and the warp scans the step's 64 rows (32 runs of 2) with
-// coalesced 128-bit loads; VT divides 32, so a lane always holds the same
-// 16-byte position of a row.  The first 8 of a lane's loads of a step are
-// issued before the step's ChaCha work; wider rows load the rest after it,
-// for 128-B rows in two halves each issued before the previous batch is
-// consumed.
-#ifndef MG_WARP_PREFETCH
-#define MG_WARP_PREFETCH 8
-#endif
+// Warp-independent fused expansion + scan.  A CTA of W warps owns a
+// contiguous range of the pass's work items, in (tile, key group) order with
+// the groups of a tile next to each other; its warps take the items one at a
+// time (ItemQueue).  Per item each lane takes one frontier node and walks its
+// 2^M leaves depth-first (stack in the warp's shared-memory slice), one leaf
+// pair per step.  Accumulators stay in registers and are flushed (warp shuffle
+// XOR) into the warp's own partial row when the group or segment changes.
+//
+// scan_pair_kernel (one key per warp; rows of 16, 32 or 64 B): a step's rows
+// are loaded before its leaf pair is expanded and stay in registers meanwhile.
+// Rows of 16 and 32 B: each lane ANDs its own pair's rows (whole sectors) with
+// its own masks.  64 B: the lanes exchange the step's 64 masks through shared
+// memory and the row loads are coalesced.  Two copies of the PRG code, one for
+// internal nodes and one for leaf pairs (about 25 KB); a third copy runs into
+// the instruction cache: 2^25 x 32 B, 3 keys 2.80 ms with three copies, 2.65
+// with one and a stack round trip per step, 2.61 with two; 2.52 with 20 warps.
+// Bound by integer issue: 89.8% of the issue slots, ALU pipe 90.8%, FMA 84.3%.
+//
+// scan_block_kernel (other row sizes, or several keys per warp): a step's rows
+// are too many for registers.  Its masks, for each of the warp's keys, go to
+// shared memory, and its 64 rows are scanned with coalesced 16-byte copies while
+// the next step's nodes are expanded: before each node expansion a chunk of the
+// earlier step's rows is copied towards shared memory (cp.async, no register
+// held), after it the chunk is used, so hardly a load is waited for and the
+// table is read at an even rate.  One copy of the PRG code, since the chunk code
+// beside it would take two past the instruction cache (no-instruction stalls
+// 0.38 per issue with two, 0.08 with one).  3 keys: 2^20 x 256 B 135 us a pass
+// (148 with the rows loaded in batches between the expansions), 10^6 x 48 B 115
+// (242 on the CTA kernel), 2^22 x 128 B 412 (475).
 
-// One depth-first step of a lane's walk: leaf pair `pi` of the lane's
-// subtree (root at tree level F, M levels deep).  The path re-joins the
-// stack (col_seed / col_t, stride 32) at relative level M - ffs(pi) (the
-// root for pi == 0), pushes the right children it passes and returns the
-// two leaf masks.
-__device__ __forceinline__ void leaf_walk(const KeyDev* __restrict__ K, const KeyAux* __restrict__ A,
-                                          uint4* col_seed, int8_t* col_t, uint32_t pi, uint32_t M, uint32_t F,
-                                          uint4& ml, uint4& mr) {
-  uint32_t lvl = pi ? (M - (uint32_t)__ffs((int)pi)) : 0u;
-  uint4 s = col_seed[lvl * 32];
-  uint32_t m = (uint32_t)(int32_t)col_t[lvl * 32];
-  for (; lvl < M - 1; ++lvl) {
-    uint4 Lc, Rc;
-    uint32_t mlc, mrc;
-    expand_cw_m(s, m, K, A, F + lvl, Lc, mlc, Rc, mrc);
-    col_seed[(lvl + 1) * 32] = Rc;
-    col_t[(lvl + 1) * 32] = (int8_t)mrc;
-    s = Lc;
-    m = mlc;
+// Stack of a lane: levels 1 .. M - 2 of its walk (stride 32 between levels).
+struct LaneStack {
+  uint4* seed;
+  int8_t* t;  // masks, one byte each (0 or 0xFF; sign-extended on load)
+};
+
+// Walk to the node of leaf pair pi (pi even) of the lane's subtree (root at
+// tree level F, M levels deep) and, when M >= 2, its sibling, the node of pair
+// pi + 1: s0, m0 and s1, m1.  For pi == 0 the caller passes the root in s0, m0;
+// otherwise the path re-joins the stack at relative level M - ffs(pi).  The
+// right children it passes are pushed, the last one staying in registers.
+__device__ __forceinline__ void walk_to_pairs(const KeyDev* __restrict__ K, const KeyAux* __restrict__ A,
+                                              const LaneStack st, const uint32_t pi, const uint32_t M,
+                                              const uint32_t F, uint4& s0, uint32_t& m0, uint4& s1, uint32_t& m1) {
+  uint32_t lvl = 0;
+  if (pi) {
+    lvl = M - (uint32_t)__ffs((int)pi);
+    s0 = st.seed[(lvl - 1) * 32];
+    m0 = (uint32_t)(int32_t)st.t[(lvl - 1) * 32];
   }
-  leaf_pair_m(s, m, A, ml, mr);
+#pragma unroll 1
+  for (; lvl + 1 < M; ++lvl) {
+    uint4 Lc;
+    uint32_t mlc;
+    expand_cw_m(s0, m0, K, A, F + lvl, Lc, mlc, s1, m1);
+    if (lvl + 2 < M) {
+      st.seed[lvl * 32] = s1;
+      st.t[lvl * 32] = (int8_t)m1;
+    }
+    s0 = Lc;
+    m0 = mlc;
+  }
 }
 
-template <int G, int VT>
-__global__ void __launch_bounds__(warp_cta_warps(G, VT) * 32, 1) scan_warp_kernel(const __grid_constant__ WarpScanParams p) {
+// 16 bytes copied to shared memory past the L1 cache, without a register.
+__device__ __forceinline__ void copy_async(uint4* dst, const uint4* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+
+// The items of a CTA's contiguous range, taken one at a time by its warps: from
+// one queue, or from four, each a quarter of the range and served by the warps
+// of one scheduler (warp w issues on scheduler w mod 4).  See WarpScanParams.
+struct ItemQueue {
+  uint64_t begin, end;
+  uint32_t* next;
+  __device__ __forceinline__ ItemQueue(const WarpScanParams& p, uint32_t* s_next, uint32_t warp, uint32_t nw) {
+    const uint32_t nq = nw < p.queues ? nw : p.queues, q = warp % nq;
+    const uint64_t b = (uint64_t)blockIdx.x * p.items / gridDim.x;
+    const uint64_t n = (uint64_t)(blockIdx.x + 1) * p.items / gridDim.x - b;
+    begin = b + n * q / nq;
+    end = b + n * (q + 1) / nq;
+    next = s_next + q;
+  }
+  __device__ __forceinline__ bool take(const uint32_t lane, uint64_t& item) const {
+    uint32_t rel = 0;
+    if (lane == 0) rel = atomicAdd(next, 1u);
+    item = begin + __shfl_sync(0xFFFFFFFFu, rel, 0);
+    return item < end;
+  }
+};
+
+__device__ __forceinline__ uint4 shfl_xor4(uint4 v, const uint32_t off) {
+  v.x ^= __shfl_xor_sync(0xFFFFFFFFu, v.x, off);
+  v.y ^= __shfl_xor_sync(0xFFFFFFFFu, v.y, off);
+  v.z ^= __shfl_xor_sync(0xFFFFFFFFu, v.z, off);
+  v.w ^= __shfl_xor_sync(0xFFFFFFFFu, v.w, off);
+  return v;
+}
+
+// Cross-block reduction at the end of a kernel: the CTA XORs its warps' partial
+// rows (written by this CTA, visible after the barrier; plain loads, not the
+// read-only path) and folds the result into the zeroed shares with 64-bit XOR
+// atomics.  XOR is associative and commutative, so the shares do not depend on
+// the order.  (The pair scan of rows up to 32 B leaves this to reduce_kernel:
+// the extra code changed its register allocation and cost 0.5% on the 31-bit
+// pass.)
+__device__ __forceinline__ void fold_partials(const WarpScanParams& p, const uint32_t nw) {
+  __syncthreads();
+  const uint4* const cta_part = p.partial + (uint64_t)blockIdx.x * nw * p.cols;
+  for (uint32_t c = threadIdx.x; c < p.cols; c += blockDim.x) {
+    uint4 v = make_uint4(0u, 0u, 0u, 0u);
+    for (uint32_t w = 0; w < nw; ++w) v = xor4(v, cta_part[(size_t)w * p.cols + c]);
+    xor_out(p.out + c, v);
+  }
+}
+
+// VT: uint4 per row (1, 2 or 4).
+template <int VT>
+__global__ void __launch_bounds__(warp_cta_warps(1) * 32, 1) scan_pair_kernel(const __grid_constant__ WarpScanParams p) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ uint32_t s_next;  // next item of this CTA's range
-  constexpr int NL = 2 * VT;            // uint4 loads per lane per step
-  constexpr int PF = NL < MG_WARP_PREFETCH ? NL : MG_WARP_PREFETCH;  // loads issued before the ChaCha work
-  constexpr uint32_t RPL = 32 / VT;     // rows covered by one warp-wide load
-  // Rows of at most 32 B with one key per warp: every lane scans
-  // its own subtree's two rows of the step (64 contiguous bytes, whole
-  // sectors) against its own leaf masks, with no shared-memory exchange and
-  // VT accumulators per key.  Wider rows use the exchange, which keeps the
-  // loads coalesced and the register count flat.
-  constexpr bool OWN = own_rows(G, VT);
+  __shared__ uint32_t s_next[4];  // next item of each scheduler's queue
+  constexpr bool OWN = VT <= 2;
+  constexpr int AV = OWN ? VT : 1;         // accumulators per lane
+  constexpr uint32_t RPL = 32 / VT;        // rows of one warp-wide load (exchange)
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   const uint32_t nw = blockDim.x >> 5;
-  const uint32_t slots = p.slots;
-  uint4* const base4 = reinterpret_cast<uint4*>(smem_raw);
-  uint4* const w_mask = base4 + (size_t)warp * G * 64;                                      // [G][64]
-  uint4* const w_seed = base4 + (size_t)nw * G * 64 + (size_t)warp * G * slots * 32;           // [G][slots][32]
-  // Stack t masks, one byte each (0 or 0xFF; sign-extended on load).
-  int8_t* const w_t = reinterpret_cast<int8_t*>(base4 + (size_t)nw * G * 64 + (size_t)nw * G * slots * 32) +
-                      (size_t)warp * G * slots * 32;
-
-  const uint64_t gw = (uint64_t)blockIdx.x * nw + warp;
-  uint4* const my_partial = p.partial + gw * p.cols;
+  const uint32_t pos = lane % VT, r0 = lane / VT;
+  // Shared memory: leaf masks [nw][64] (exchange only), stacks [nw][slots][32],
+  // then the stacks' t masks.
+  constexpr uint32_t nm = OWN ? 0u : 64u;
+  uint4* const w_mask = reinterpret_cast<uint4*>(smem_raw) + (size_t)warp * nm;
+  uint4* const stk4 = reinterpret_cast<uint4*>(smem_raw) + (size_t)nw * nm;
+  const LaneStack st = {stk4 + (size_t)warp * p.slots * 32 + lane,
+                        reinterpret_cast<int8_t*>(stk4 + (size_t)nw * p.slots * 32) + (size_t)warp * p.slots * 32 + lane};
+  uint4* const my_partial = p.partial + ((uint64_t)blockIdx.x * nw + warp) * p.cols;
   for (uint32_t c = lane; c < p.cols; c += 32) my_partial[c] = make_uint4(0u, 0u, 0u, 0u);
-  const uint64_t c_begin = (uint64_t)blockIdx.x * p.items / gridDim.x;
-  const uint64_t c_end = (uint64_t)(blockIdx.x + 1) * p.items / gridDim.x;
-  if (threadIdx.x == 0) s_next = 0;
+  const ItemQueue queue(p, s_next, warp, nw);
+  if (threadIdx.x < 4) s_next[threadIdx.x] = 0;
   __syncthreads();
 
-  const uint32_t pos = lane % VT, r0 = lane / VT;
-  constexpr int AV = OWN ? VT : 1;
-  uint4 acc[G];
-  uint4 own[G][AV];
+  uint4 acc[AV];
 #pragma unroll
-  for (int k = 0; k < G; ++k) {
-    acc[k] = make_uint4(0u, 0u, 0u, 0u);
-#pragma unroll
-    for (int v = 0; v < AV; ++v) own[k][v] = make_uint4(0u, 0u, 0u, 0u);
-  }
+  for (int v = 0; v < AV; ++v) acc[v] = make_uint4(0u, 0u, 0u, 0u);
   int cur_seg = -1;
   uint32_t cur_group = 0;
-
-  auto flush_own = [&](const WarpSeg& sg, uint32_t group) {
-#pragma unroll
-    for (int k = 0; k < G; ++k) {
-#pragma unroll
-      for (int v = 0; v < AV; ++v) {
-        uint4 x = own[k][v];
-#pragma unroll
-        for (uint32_t off = 16; off >= 1; off >>= 1) {
-          x.x ^= __shfl_xor_sync(0xFFFFFFFFu, x.x, off);
-          x.y ^= __shfl_xor_sync(0xFFFFFFFFu, x.y, off);
-          x.z ^= __shfl_xor_sync(0xFFFFFFFFu, x.z, off);
-          x.w ^= __shfl_xor_sync(0xFFFFFFFFu, x.w, off);
-        }
-        if ((uint32_t)k < sg.g && lane == (uint32_t)v) {
-          const size_t col = sg.col_base + ((size_t)group * sg.g + k) * VT + v;
-          my_partial[col] = xor4(my_partial[col], x);
-        }
-        own[k][v] = make_uint4(0u, 0u, 0u, 0u);
-      }
-    }
-  };
-
   auto flush = [&](const WarpSeg& sg, uint32_t group) {
-    if constexpr (OWN) {
-      flush_own(sg, group);
-      return;
-    }
 #pragma unroll
-    for (int k = 0; k < G; ++k) {
-      uint4 v = acc[k];
+    for (int v = 0; v < AV; ++v) {
+      uint4 x = acc[v];
 #pragma unroll
-      for (uint32_t off = 16; off >= (uint32_t)VT; off >>= 1) {
-        v.x ^= __shfl_xor_sync(0xFFFFFFFFu, v.x, off);
-        v.y ^= __shfl_xor_sync(0xFFFFFFFFu, v.y, off);
-        v.z ^= __shfl_xor_sync(0xFFFFFFFFu, v.z, off);
-        v.w ^= __shfl_xor_sync(0xFFFFFFFFu, v.w, off);
+      for (uint32_t off = 16; off >= (OWN ? 1u : (uint32_t)VT); off >>= 1) x = shfl_xor4(x, off);
+      if (OWN ? lane == (uint32_t)v : lane < (uint32_t)VT) {
+        const size_t col = sg.col_base + (size_t)group * VT + (OWN ? (uint32_t)v : lane);
+        my_partial[col] = xor4(my_partial[col], x);
       }
-      if ((uint32_t)k < sg.g && lane < (uint32_t)VT) {
-        const size_t col = sg.col_base + ((size_t)group * sg.g + k) * VT + lane;
-        my_partial[col] = xor4(my_partial[col], v);
-      }
-      acc[k] = make_uint4(0u, 0u, 0u, 0u);
+      acc[v] = make_uint4(0u, 0u, 0u, 0u);
     }
   };
 
-
-  for (;;) {
-    uint32_t rel = 0;
-    if (lane == 0) rel = atomicAdd(&s_next, 1u);
-    rel = __shfl_sync(0xFFFFFFFFu, rel, 0);
-    const uint64_t item = c_begin + rel;
-    if (item >= c_end) break;
+  for (uint64_t item; queue.take(lane, item);) {
     uint32_t si = 0;
     while (si + 1 < p.nsegs && item >= p.seg[si + 1].item_begin) ++si;
     const WarpSeg& sg = p.seg[si];
@@ -499,195 +514,318 @@ __global__ void __launch_bounds__(warp_cta_warps(G, VT) * 32, 1) scan_warp_kerne
       cur_seg = (int)si;
       cur_group = group;
     }
-    const uint32_t g = sg.g, M = sg.M;
-    const uint32_t F = sg.d - M;
+    const uint32_t M = sg.M, F = sg.d - M;
     const uint64_t node = (uint64_t)tile * 32 + lane;
     const bool valid = node < sg.nF;
-    const KeyDev* __restrict__ kp = p.keys + sg.key_base + (size_t)group * g;
-    const KeyAux* __restrict__ ap = p.aux + sg.key_base + (size_t)group * g;
-    for (uint32_t k = 0; k < g; ++k) {
-      const uint64_t idx = sg.fr_base + ((uint64_t)group * g + k) * sg.nF + node;
-      w_seed[(k * slots) * 32 + lane] = valid ? p.fr_seed[idx] : make_uint4(0u, 0u, 0u, 0u);
-      w_t[(k * slots) * 32 + lane] = (valid && p.fr_t[idx] == 1) ? (int8_t)-1 : (int8_t)0;
-    }
+    const KeyDev* __restrict__ K = p.keys + sg.key_base + group;
+    const KeyAux* __restrict__ A = p.aux + sg.key_base + group;
+    const uint64_t idx = sg.fr_base + (uint64_t)group * sg.nF + node;
+    uint4 s0 = valid ? p.fr_seed[idx] : make_uint4(0u, 0u, 0u, 0u);
+    uint32_t m0 = (valid && p.fr_t[idx] == 1) ? 0xFFFFFFFFu : 0u;
     const uint4* __restrict__ tbl = sg.table;
     const uint64_t nrows = sg.rows;
     // Table row of the warp tile's first leaf (wraps below the first row).
     const uint64_t row0 = (((sg.first >> M) + (uint64_t)tile * 32) << M) - sg.first;
     const uint32_t pairs = 1u << (M - 1);
-    // A warp tile whose 32 x 2^M rows all lie in the table takes the
-    // unchecked path: per-lane row pointers advance by one leaf pair per step
-    // (load jj of a step is RPL / 2 producing lanes further on; RPL is even
-    // for rows up to 256 B).
+    // A warp tile whose 32 x 2^M rows all lie in the table needs no bounds checks.
     const bool full = row0 < nrows && nrows - row0 >= ((uint64_t)32 << M);
-    const uint4* const lp = full ? tbl + (row0 + ((uint64_t)(r0 >> 1) << M) + (r0 & 1u)) * VT + pos : tbl;
-    const size_t jstride = ((size_t)(RPL >> 1) << M) * VT;
-    // Own-rows path: the lane's first row of the tile (its subtree's leaves).
-    const uint4* const own_lp = full ? tbl + (row0 + ((uint64_t)lane << M)) * VT : tbl;
-    auto run_own = [&](auto full_tag) {
-    constexpr bool FULL = decltype(full_tag)::value;
-    for (uint32_t pi = 0; pi < pairs; pi += 2) {
-      // Walk to the node of leaf pair pi and, when M >= 2, its sibling, the
-      // node of pair pi + 1: the path re-joins the stack at relative level
-      // M - ffs(pi) (the root for pi == 0) and pushes the right children it
-      // passes, the last one staying in registers.
-      uint32_t lvl = pi ? (M - (uint32_t)__ffs((int)pi)) : 0u;
-      uint4 s0 = w_seed[lvl * 32 + lane], s1 = make_uint4(0u, 0u, 0u, 0u);
-      uint32_t m0 = (uint32_t)(int32_t)w_t[lvl * 32 + lane], m1 = 0u;
-#pragma unroll 1
-      for (; lvl + 1 < M; ++lvl) {
-        uint32_t mlc;
-        uint4 Lc;
-        expand_cw_m(s0, m0, kp, ap, F + lvl, Lc, mlc, s1, m1);
-        if (lvl + 2 < M) {
-          w_seed[(lvl + 1) * 32 + lane] = s1;
-          w_t[(lvl + 1) * 32 + lane] = (int8_t)m1;
-        }
-        s0 = Lc;
-        m0 = mlc;
-      }
-#pragma unroll 1
-      for (uint32_t h = 0; h < 2u && pi + h < pairs; ++h) {
-        uint4 dat[2 * AV];
-#pragma unroll
-        for (int j = 0; j < 2 * AV; ++j) {
-          if constexpr (FULL) {
-            dat[j] = __ldg(own_lp + (size_t)(pi + h) * (2 * VT) + j);
-          } else {
-            const uint64_t row = row0 + ((uint64_t)lane << M) + 2u * (pi + h) + (uint32_t)(j / AV);
-            dat[j] = row < nrows ? __ldg(tbl + row * VT + (j % AV)) : make_uint4(0u, 0u, 0u, 0u);
-          }
-        }
-        uint4 ml, mr;
-        leaf_pair_m(s0, m0, ap, ml, mr);
-#pragma unroll
-        for (int v = 0; v < AV; ++v) {
-          own[0][v] = xor_and(own[0][v], dat[v], ml);
-          own[0][v] = xor_and(own[0][v], dat[AV + v], mr);
-        }
-        s0 = s1;
-        m0 = m1;
-      }
-    }
+    // Row of load j of a step: the lane's own pair, or row r = r0 + j * RPL of
+    // the warp's 64 (leaf r mod 2 of lane r / 2; RPL is even).
+    auto row_of = [&](int j) {
+      return OWN ? ((uint64_t)lane << M) + (uint32_t)(j / VT)
+                 : ((uint64_t)((r0 + (uint32_t)j * RPL) >> 1) << M) + (r0 & 1u);
     };
-    auto run_steps = [&](auto full_tag) {
-    constexpr bool FULL = decltype(full_tag)::value && (RPL % 2 == 0);
-    for (uint32_t pi = 0; pi < pairs; ++pi) {
-      // Rows of this step: r = 2 * (producing lane) + leaf.
-      uint4 dat[PF > 0 ? PF : 1];
-#pragma unroll
-      for (int jj = 0; jj < PF; ++jj) {
-        const uint32_t r = r0 + (uint32_t)jj * RPL;
-        const uint64_t row = row0 + ((uint64_t)(r >> 1) << M) + 2u * pi + (r & 1u);
-        if constexpr (FULL) {
-          (void)row;
-          dat[jj] = __ldg(lp + (size_t)pi * (2 * VT) + (size_t)jj * jstride);
-        } else {
-          dat[jj] = row < nrows ? __ldg(tbl + row * VT + pos) : make_uint4(0u, 0u, 0u, 0u);
-        }
-      }
+    const uint4* const lp = full ? tbl + (row0 + row_of(0)) * VT + (OWN ? 0u : pos) : tbl;
+    const size_t jstep = ((size_t)(RPL >> 1) << M) * VT;  // exchange: from load j to j + 1
+    auto run = [&](auto full_tag) {
+      constexpr bool FULL = decltype(full_tag)::value;
+      for (uint32_t pi = 0; pi < pairs; pi += 2) {
+        uint4 s1 = make_uint4(0u, 0u, 0u, 0u);
+        uint32_t m1 = 0u;
+        walk_to_pairs(K, A, st, pi, M, F, s0, m0, s1, m1);
 #pragma unroll 1
-      for (uint32_t k = 0; k < g; ++k) {
-        uint4 ml, mr;
-        leaf_walk(kp + k, ap + k, w_seed + (size_t)k * slots * 32 + lane, w_t + (size_t)k * slots * 32 + lane,
-                  pi, M, F, ml, mr);
-        w_mask[k * 64 + 2 * lane] = ml;
-        w_mask[k * 64 + 2 * lane + 1] = mr;
-      }
-      __syncwarp();
-      auto load_rows = [&](uint4* buf, int j0, auto n_tag) {
-        constexpr int N = decltype(n_tag)::value;
+        for (uint32_t h = 0; h < 2u && pi + h < pairs; ++h) {
+          // The step's rows, loaded before the ChaCha work.
+          uint4 dat[2 * VT];
 #pragma unroll
-        for (int jj = 0; jj < N; ++jj) {
-          const uint32_t r = r0 + (uint32_t)(j0 + jj) * RPL;
-          const uint64_t row = row0 + ((uint64_t)(r >> 1) << M) + 2u * pi + (r & 1u);
-          if constexpr (FULL) {
-            (void)row;
-            buf[jj] = __ldg(lp + (size_t)pi * (2 * VT) + (size_t)(j0 + jj) * jstride);
-          } else {
-            buf[jj] = row < nrows ? __ldg(tbl + row * VT + pos) : make_uint4(0u, 0u, 0u, 0u);
+          for (int j = 0; j < 2 * VT; ++j) {
+            if constexpr (FULL) {
+              dat[j] = __ldg(lp + (size_t)(pi + h) * (2 * VT) + (OWN ? (size_t)j : (size_t)j * jstep));
+            } else {
+              const uint64_t row = row0 + row_of(j) + 2u * (pi + h);
+              dat[j] = row < nrows ? __ldg(tbl + row * VT + (OWN ? (uint32_t)(j % VT) : pos))
+                                   : make_uint4(0u, 0u, 0u, 0u);
+            }
           }
-        }
-      };
-      auto use_rows = [&](const uint4* buf, int j0, auto n_tag) {
-        constexpr int N = decltype(n_tag)::value;
+          uint4 ml, mr;
+          leaf_pair_m(s0, m0, A, ml, mr);
+          if constexpr (OWN) {
 #pragma unroll
-        for (int jj = 0; jj < N; ++jj) {
-          const uint32_t r = r0 + (uint32_t)(j0 + jj) * RPL;
+            for (int v = 0; v < AV; ++v) {
+              acc[v] = xor_and(acc[v], dat[v], ml);
+              acc[v] = xor_and(acc[v], dat[VT + v], mr);
+            }
+          } else {
+            w_mask[2 * lane] = ml;
+            w_mask[2 * lane + 1] = mr;
+            __syncwarp();
 #pragma unroll
-          for (int k = 0; k < G; ++k)
-            if ((uint32_t)k < g) acc[k] = xor_and(acc[k], buf[jj], w_mask[k * 64 + r]);
-        }
-      };
-      // The rest of the step's loads (the ChaCha registers are free now).
-      // 128-B rows: two halves, each issued before the previous batch is
-      // consumed.  Wider rows: chunks of 8 (holding more of them in flight
-      // makes the kernel spill).
-      constexpr int REST = NL - PF;
-      if constexpr (REST == 0) {
-        use_rows(dat, 0, std::integral_constant<int, PF>{});
-      } else if constexpr (REST <= 8) {
-        constexpr int H = REST / 2 > 0 ? (REST % 2 == 0 ? REST / 2 : REST) : REST;
-        uint4 ma[H];
-        load_rows(ma, PF, std::integral_constant<int, H>{});
-        use_rows(dat, 0, std::integral_constant<int, PF>{});
-        if constexpr (H < REST) {
-          uint4 mb[REST - H];
-          load_rows(mb, PF + H, std::integral_constant<int, REST - H>{});
-          use_rows(ma, PF, std::integral_constant<int, H>{});
-          use_rows(mb, PF + H, std::integral_constant<int, REST - H>{});
-        } else {
-          use_rows(ma, PF, std::integral_constant<int, H>{});
-        }
-      } else {
-        use_rows(dat, 0, std::integral_constant<int, PF>{});
-        constexpr int CH2 = 8;
-        static_assert(REST % CH2 == 0, "load chunks must tile the step");
-#pragma unroll 1
-        for (int j0 = PF; j0 < NL; j0 += CH2) {
-          uint4 more[CH2];
-          load_rows(more, j0, std::integral_constant<int, CH2>{});
-          use_rows(more, j0, std::integral_constant<int, CH2>{});
+            for (int j = 0; j < 2 * VT; ++j) acc[0] = xor_and(acc[0], dat[j], w_mask[r0 + (uint32_t)j * RPL]);
+            __syncwarp();
+          }
+          s0 = s1;
+          m0 = m1;
         }
       }
-      __syncwarp();
-    }
     };
-    if constexpr (OWN) {
-      if (full)
-        run_own(std::true_type{});
-      else
-        run_own(std::false_type{});
-    } else {
-      if (full)
-        run_steps(std::true_type{});
-      else
-        run_steps(std::false_type{});
-    }
+    if (full)
+      run(std::true_type{});
+    else
+      run(std::false_type{});
   }
   if (cur_seg >= 0) flush(p.seg[cur_seg], cur_group);
-  if constexpr (!OWN) {
-    // Cross-block reduction of the wide-row instantiations: the CTA XORs its
-    // warps' partial rows (written by this CTA, visible after the barrier;
-    // plain loads, not the read-only path) and folds the result into the
-    // zeroed shares with 64-bit XOR atomics.  XOR is associative and
-    // commutative, so the shares do not depend on the order.  (The own-rows
-    // instantiations leave this to reduce_kernel: the extra code changes
-    // their register allocation and costs 0.5% on the 31-bit pass, far more
-    // than the reduction launch it saves.)
-    __syncthreads();
-    const uint4* const cta_part = p.partial + (uint64_t)blockIdx.x * nw * p.cols;
-    for (uint32_t c = threadIdx.x; c < p.cols; c += blockDim.x) {
-      uint4 v = make_uint4(0u, 0u, 0u, 0u);
-      for (uint32_t w = 0; w < nw; ++w) v = xor4(v, cta_part[(size_t)w * p.cols + c]);
-      xor_out(p.out + c, v);
-    }
-  }
+  if constexpr (!OWN) fold_partials(p, nw);
 }
 
-// Whether scan_warp_kernel<G, VT> reduces its partial rows into the shares
-// itself (wide rows) or leaves them to reduce_kernel (own-rows scan).
-bool warp_reduces_in_kernel(int G, uint32_t VT) { return !own_rows(G, VT); }
+// VT: uint4 per row when it is a power of two (4..32), 0 for any other V up to
+// 32 (p.V).  RPL = 32 / V rows are covered by one warp-wide load; V * RPL
+// lanes take part and a lane always holds the same 16-byte position of a row.
+// Row r of a step (0..63) is leaf r mod 2 of lane r / 2; its mask lies at
+// r ^ ((r >> 3) mod 2), so that the lanes' stores of one leaf and the loads of
+// consecutive rows both touch all banks.
+template <int G, int VT>
+__global__ void __launch_bounds__(warp_cta_warps(G) * 32, 1)
+    scan_block_kernel(const __grid_constant__ WarpScanParams p) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ uint32_t s_next[4];  // next item of each scheduler's queue
+  constexpr uint32_t kRows = 32u * kBlockLeaves;
+  constexpr int CH = block_chunk(VT);  // loads per lane and chunk
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const uint32_t nw = blockDim.x >> 5;
+  const uint32_t V = VT ? (uint32_t)VT : p.V;
+  const uint32_t RPL = 32u / V;
+  const uint32_t pos = lane % V, r0 = lane / V;
+  const bool scans = VT ? true : lane < V * RPL;
+  const uint32_t nload = (kRows + RPL - 1) / RPL;  // loads per lane and block
+  // Shared memory: masks of two blocks [nw][2][G][kRows], stacks
+  // [nw][G][slots][32], then the stacks' t masks.
+  constexpr uint32_t nm = 2u * G * kRows;
+  const uint32_t ns = G * p.slots * 32u;
+  uint4* const sm4 = reinterpret_cast<uint4*>(smem_raw);
+  uint4* const w_mask = sm4 + (size_t)warp * nm;
+  uint4* const w_stage = sm4 + (size_t)nw * nm + (size_t)warp * CH * 32 + lane;
+  uint4* const w_stk = sm4 + (size_t)nw * (nm + CH * 32) + (size_t)warp * ns + lane;
+  int8_t* const w_stk_t = reinterpret_cast<int8_t*>(sm4 + (size_t)nw * (nm + CH * 32 + ns)) + (size_t)warp * ns + lane;
+
+  uint4* const my_partial = p.partial + ((uint64_t)blockIdx.x * nw + warp) * p.cols;
+  for (uint32_t c = lane; c < p.cols; c += 32) my_partial[c] = make_uint4(0u, 0u, 0u, 0u);
+  const ItemQueue queue(p, s_next, warp, nw);
+  if (threadIdx.x < 4) s_next[threadIdx.x] = 0;
+  __syncthreads();
+
+  uint4 acc[G];
+#pragma unroll
+  for (int k = 0; k < G; ++k) acc[k] = make_uint4(0u, 0u, 0u, 0u);
+  int cur_seg = -1;
+  uint32_t cur_group = 0, M = 2;
+
+  // Load j of a lane is row r = r0 + j * RPL of the block, off(r) rows below
+  // its first row, with its mask at mask_at(r).  When V is a power of two the
+  // bits of r0 and j * RPL are disjoint and both maps split into a lane part
+  // (r0) and a part of j that is the same for all lanes.
+  auto row_off = [&](uint32_t r) { return ((r / kBlockLeaves) << M) + r % kBlockLeaves; };
+  auto mask_at = [&](uint32_t r) { return r ^ ((r >> 3) % kBlockLeaves); };
+  const uint32_t lane_mask = mask_at(r0);
+  auto use_rows = [&](const uint4* masks, const uint4* stage, uint32_t j0) {
+#pragma unroll
+    for (int j = 0; j < CH; ++j) {
+      uint32_t at;
+      if constexpr (VT != 0) {
+        at = lane_mask ^ mask_at(j0 * RPL) ^ mask_at((uint32_t)j * RPL);
+      } else {
+        const uint32_t r = r0 + (j0 + (uint32_t)j) * RPL;
+        at = mask_at(r < kRows ? r : kRows - 1u);  // past the block the data is zero
+      }
+      const uint4 row = stage[j * 32];
+#pragma unroll
+      for (int k = 0; k < G; ++k) acc[k] = xor_and(acc[k], row, masks[k * kRows + at]);
+    }
+  };
+
+  // The step whose rows are being scanned (all of them in the table): its rows
+  // are copied a chunk at a time before, and used after, the node expansions of
+  // the next step.
+  const uint4* pend_row = nullptr;    // the lane's row 0
+  const uint4* pend_mask = w_mask;
+  uint32_t pend_j = nload;            // next load; nload: nothing pending
+  uint32_t buf_at = 0;                // mask buffer of the next step
+  auto load_chunk = [&]() {
+    if (pend_j >= nload) return;
+    if constexpr (VT != 0) {
+      const uint4* const q = pend_row + (size_t)row_off(pend_j * RPL) * V;
+#pragma unroll
+      for (int j = 0; j < CH; ++j) copy_async(w_stage + j * 32, q + row_off((uint32_t)j * RPL) * V);
+    } else {
+#pragma unroll
+      for (int j = 0; j < CH; ++j) {
+        const uint32_t r = r0 + (pend_j + (uint32_t)j) * RPL;
+        if (scans && r < kRows)
+          copy_async(w_stage + j * 32, pend_row + (size_t)row_off(r) * V);
+        else
+          w_stage[j * 32] = make_uint4(0u, 0u, 0u, 0u);
+      }
+    }
+  };
+  auto use_chunk = [&]() {
+    if (pend_j >= nload) return;
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    use_rows(pend_mask, w_stage, pend_j);
+    pend_j += CH;
+  };
+  auto drain = [&]() {
+#pragma unroll 1
+    while (pend_j < nload) {
+      load_chunk();
+      use_chunk();
+    }
+  };
+  auto flush = [&](const WarpSeg& sg, uint32_t group) {
+#pragma unroll
+    for (int k = 0; k < G; ++k) {
+      uint4 v = acc[k];
+      if constexpr (VT != 0) {
+#pragma unroll
+        for (uint32_t off = 16; off >= (uint32_t)VT; off >>= 1) v = shfl_xor4(v, off);
+      } else {
+        const uint4 x = v;
+        for (uint32_t i = 1; i < RPL; ++i) {
+          const uint32_t src = (lane + i * V) & 31u;
+          v.x ^= __shfl_sync(0xFFFFFFFFu, x.x, src);
+          v.y ^= __shfl_sync(0xFFFFFFFFu, x.y, src);
+          v.z ^= __shfl_sync(0xFFFFFFFFu, x.z, src);
+          v.w ^= __shfl_sync(0xFFFFFFFFu, x.w, src);
+        }
+      }
+      if ((uint32_t)k < sg.g && lane < V) {
+        const size_t col = sg.col_base + ((size_t)group * sg.g + k) * V + lane;
+        my_partial[col] = xor4(my_partial[col], v);
+      }
+      acc[k] = make_uint4(0u, 0u, 0u, 0u);
+    }
+  };
+
+  for (uint64_t item; queue.take(lane, item);) {
+    uint32_t si = 0;
+    while (si + 1 < p.nsegs && item >= p.seg[si + 1].item_begin) ++si;
+    const WarpSeg& sg = p.seg[si];
+    const uint64_t local = item - sg.item_begin;
+    const uint32_t tile = (uint32_t)(local / sg.groups);
+    const uint32_t group = (uint32_t)(local % sg.groups);
+    const uint32_t g = sg.g;
+    if ((int)si != cur_seg || group != cur_group) {
+      if (cur_seg >= 0) {
+        drain();
+        flush(p.seg[cur_seg], cur_group);
+      }
+      // A segment of fewer than G keys: the other keys' masks are zero, so the
+      // row scan needs no test of the key count.
+      if ((int)si != cur_seg) {
+        __syncwarp();
+        for (uint32_t i = lane; i < nm; i += 32) w_mask[i] = make_uint4(0u, 0u, 0u, 0u);
+        __syncwarp();
+      }
+      cur_seg = (int)si;
+      cur_group = group;
+      M = sg.M;
+    }
+    const uint32_t F = sg.d - M;
+    const uint64_t node = (uint64_t)tile * 32 + lane;
+    const bool valid = node < sg.nF;
+    const KeyDev* __restrict__ kp = p.keys + sg.key_base + (size_t)group * g;
+    const KeyAux* __restrict__ ap = p.aux + sg.key_base + (size_t)group * g;
+    // A key's root waits in its stack's first slot, which level 1 takes over
+    // once the walk has read it.
+    for (uint32_t k = 0; k < g; ++k) {
+      const uint64_t idx = sg.fr_base + ((uint64_t)group * g + k) * sg.nF + node;
+      w_stk[k * p.slots * 32] = valid ? p.fr_seed[idx] : make_uint4(0u, 0u, 0u, 0u);
+      w_stk_t[k * p.slots * 32] = (valid && p.fr_t[idx] == 1) ? (int8_t)-1 : (int8_t)0;
+    }
+    const uint4* __restrict__ tbl = sg.table;
+    const uint64_t nrows = sg.rows;
+    // Table row of the warp tile's first leaf (wraps below the first row).
+    const uint64_t row0 = (((sg.first >> M) + (uint64_t)tile * 32) << M) - sg.first;
+    // A warp tile whose 32 x 2^M rows all lie in the table needs no bounds
+    // checks.  (Depth 1 has no second pair and takes the checked path.)
+    const bool full = row0 < nrows && nrows - row0 >= ((uint64_t)32 << M);
+    const uint32_t pairs = 1u << (M - 1);
+    for (uint32_t pi = 0; pi < pairs; ++pi) {
+      // The step's masks, key by key.
+      uint4* const masks = w_mask + buf_at * (G * kRows);
+#pragma unroll 1
+      for (uint32_t k = 0; k < g; ++k) {
+        uint4* const st_seed = w_stk + k * p.slots * 32;
+        int8_t* const st_t = w_stk_t + k * p.slots * 32;
+        const KeyDev* __restrict__ K = kp + k;
+        const KeyAux* __restrict__ A = ap + k;
+        uint32_t lvl = pi ? M - (uint32_t)__ffs((int)pi) : 0u;
+        uint4 s = st_seed[(pi ? lvl - 1 : 0u) * 32];
+        uint32_t m = (uint32_t)(int32_t)st_t[(pi ? lvl - 1 : 0u) * 32];
+        for (bool leaf = false; !leaf;) {
+          load_chunk();
+          uint4 Lc, Rc;
+          uint32_t bl, br;
+          prg_expand(s, Lc, Rc, bl, br);
+          leaf = lvl + 1 >= M;
+          if (!leaf) {
+            uint32_t mr;
+            apply_cw_m(Lc, Rc, bl, br, m, K, A, F + lvl, m, mr);
+            st_seed[lvl * 32] = Rc;
+            st_t[lvl * 32] = (int8_t)mr;
+            s = Lc;
+            ++lvl;
+          } else {
+            uint4 ml, mr;
+            leaf_terms_m(Lc, Rc, bl, br, m, A, ml, mr);
+            masks[k * kRows + mask_at(lane * 2u)] = ml;
+            masks[k * kRows + mask_at(lane * 2u + 1u)] = mr;
+          }
+          use_chunk();
+        }
+      }
+      drain();
+      __syncwarp();  // the masks are written, and the other buffer's are read
+      const uint64_t blk_row0 = row0 + 2u * pi;
+      if (full) {
+        pend_row = tbl + (blk_row0 + (VT ? row_off(r0) : 0u)) * V + pos;
+        pend_mask = masks;
+        pend_j = 0;
+        buf_at ^= 1u;
+      } else {
+#pragma unroll 1
+        for (uint32_t j0 = 0; j0 < nload; j0 += CH) {
+#pragma unroll
+          for (int j = 0; j < CH; ++j) {
+            const uint32_t r = r0 + (j0 + (uint32_t)j) * RPL;
+            const uint64_t row = blk_row0 + row_off(r);
+            const bool in = scans && r < kRows && row < nrows;
+            w_stage[j * 32] = in ? __ldg(tbl + row * V + pos) : make_uint4(0u, 0u, 0u, 0u);
+          }
+          use_rows(masks, w_stage, j0);
+        }
+        __syncwarp();
+      }
+    }
+  }
+  if (cur_seg >= 0) {
+    drain();
+    flush(p.seg[cur_seg], cur_group);
+  }
+  fold_partials(p, nw);
+}
+
+// Whether the warp kernel reduces its partial rows into the shares itself
+// or leaves them to reduce_kernel (the pair scan of rows up to 32 B).
+bool warp_reduces_in_kernel(int G, uint32_t V) { return G > 1 || V > 2; }
 
 // out[c] ^= XOR over the nparts partial rows (launch_reduce zeroes out first).
 // Block (x, y) = cpb columns x (kThreads / cpb) slices over the partial rows
@@ -1027,64 +1165,60 @@ cudaError_t launch_eval_points(const KeyDev* key, const uint64_t* idx, uint64_t 
 
 // ---- warp-path launchers --------------------------------------------------
 
-// Dynamic shared memory of a warp-kernel CTA of nw warps: per warp, G keys'
-// leaf-mask exchange buffers and depth-first stacks.
-size_t warp_smem_bytes(int G, uint32_t VT, uint32_t slots, uint32_t nw) {
-  (void)VT;
-  return (size_t)nw * G * (64 * 16 + (size_t)slots * 32 * 17);
+// Levels of a lane's stack: 1 .. M - 2 (the last right child stays in
+// registers); the block scan keeps a key's root in the first slot too.
+uint32_t warp_slots(int G, uint32_t V, uint32_t M) { const uint32_t top = pair_scan(G, V) ? 2 : 1; return M > top ? M - top : 1; }
+
+// Dynamic shared memory of a warp-kernel CTA of nw warps.  Own-rows scan: a
+// stack per warp.  Block scan: two blocks of masks and a stack per key and warp.
+size_t warp_smem_bytes(int G, uint32_t V, uint32_t slots, uint32_t nw) {
+  if (pair_scan(G, V)) return (size_t)nw * 32 * ((V > 2 ? 2 * 16 : 0) + (size_t)slots * 17);
+  return (size_t)nw * 32 * ((size_t)block_chunk(V) * 16 + (size_t)G * (2 * kBlockLeaves * 16 + (size_t)slots * 17));
 }
 
-bool warp_vt_supported(uint32_t V) { return V == 1 || V == 2 || V == 4 || V == 8 || V == 16 || V == 32; }
+bool warp_vt_supported(uint32_t V) { return V >= 1 && V <= 32; }
 
-template <int G, int VT>
-static cudaError_t warp_prepare_t(size_t smem) {
-  return raise_smem_limit(reinterpret_cast<const void*>(scan_warp_kernel<G, VT>), smem);
-}
-template <int G, int VT>
-static int warp_occupancy_t(size_t smem, uint32_t nw) {
-  int n = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, scan_warp_kernel<G, VT>, (int)(nw * 32), smem) != cudaSuccess)
-    return 0;
-  return n;
-}
-template <int G, int VT>
-static cudaError_t warp_launch_t(const WarpScanParams& p, uint32_t grid, uint32_t nw, size_t smem, cudaStream_t st) {
-  scan_warp_kernel<G, VT><<<grid, nw * 32, smem, st>>>(p);
-  return cudaGetLastError();
-}
-
-#define MG_VT_DISPATCH(G_, VT_, FN, ...)                \
-  switch (VT_) {                                        \
-    case 1: return FN<G_, 1>(__VA_ARGS__);              \
-    case 2: return FN<G_, 2>(__VA_ARGS__);              \
-    case 4: return FN<G_, 4>(__VA_ARGS__);              \
-    case 8: return FN<G_, 8>(__VA_ARGS__);              \
-    case 16: return FN<G_, 16>(__VA_ARGS__);            \
-    case 32: return FN<G_, 32>(__VA_ARGS__);            \
-    default: break;                                     \
+using WarpKernel = void (*)(const WarpScanParams);
+template <int G>
+static WarpKernel block_kernel(uint32_t V) {
+  switch (V) {
+    case 4: return scan_block_kernel<G, 4>;
+    case 8: return scan_block_kernel<G, 8>;
+    case 16: return scan_block_kernel<G, 16>;
+    case 32: return scan_block_kernel<G, 32>;
+    default: return scan_block_kernel<G, 0>;
   }
-
-#define MG_GVT_DISPATCH(G, VT, FN, FAIL, ...)                 \
-  switch (G) {                                                \
-    case 1: MG_VT_DISPATCH(1, VT, FN, __VA_ARGS__) break;     \
-    case 2: MG_VT_DISPATCH(2, VT, FN, __VA_ARGS__) break;     \
-    case 3: MG_VT_DISPATCH(3, VT, FN, __VA_ARGS__) break;     \
-    case 4: MG_VT_DISPATCH(4, VT, FN, __VA_ARGS__) break;     \
-    default: break;                                           \
-  }                                                           \
-  return FAIL;
+}
+static WarpKernel warp_kernel(int G, uint32_t V) {
+  if (!warp_vt_supported(V)) return nullptr;
+  if (pair_scan(G, V)) return V == 1 ? scan_pair_kernel<1> : V == 2 ? scan_pair_kernel<2> : scan_pair_kernel<4>;
+  switch (G) {
+    case 1: return block_kernel<1>(V);
+    case 2: return block_kernel<2>(V);
+    case 3: return block_kernel<3>(V);
+    case 4: return block_kernel<4>(V);
+    default: return nullptr;
+  }
+}
 
 bool warp_g_supported(int G) { return G >= 1 && G <= 4; }
 
-cudaError_t warp_prepare(int G, uint32_t VT, size_t smem) {
-  MG_GVT_DISPATCH(G, VT, warp_prepare_t, cudaErrorInvalidValue, smem)
+cudaError_t warp_prepare(int G, uint32_t V, size_t smem) {
+  const WarpKernel k = warp_kernel(G, V);
+  return k ? raise_smem_limit(reinterpret_cast<const void*>(k), smem) : cudaErrorInvalidValue;
 }
-int warp_occupancy(int G, uint32_t VT, size_t smem, uint32_t nw) {
-  MG_GVT_DISPATCH(G, VT, warp_occupancy_t, 0, smem, nw)
+int warp_occupancy(int G, uint32_t V, size_t smem, uint32_t nw) {
+  const WarpKernel k = warp_kernel(G, V);
+  int n = 0;
+  if (!k || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, (int)(nw * 32), smem) != cudaSuccess) return 0;
+  return n;
 }
-cudaError_t launch_scan_warp(int G, uint32_t VT, const WarpScanParams& p, uint32_t grid, uint32_t nw, size_t smem,
+cudaError_t launch_scan_warp(int G, uint32_t V, const WarpScanParams& p, uint32_t grid, uint32_t nw, size_t smem,
                              cudaStream_t st) {
-  MG_GVT_DISPATCH(G, VT, warp_launch_t, cudaErrorInvalidValue, p, grid, nw, smem, st)
+  const WarpKernel k = warp_kernel(G, V);
+  if (!k) return cudaErrorInvalidValue;
+  k<<<grid, nw * 32, smem, st>>>(p);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_delta(const KeyDev* keys, const uint2* jobs, uint32_t njobs, const uint64_t* idx,

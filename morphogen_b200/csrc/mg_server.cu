@@ -56,15 +56,21 @@ struct Request {
 };
 
 // Device bytes a key adds to a pass: its device copy (key and warp-kernel
-// constants, 1200 B), its frontier (17 B per
-// node: at most rows / 2 nodes for tables up to 2^24 rows, rows / 2^8 above,
-// where the planner keeps at least 8 depth-first levels) and partial-row
-// columns for every persistent warp.
+// constants, 1264 B), its frontier (17 B per node: at most rows / 2 nodes for
+// tables up to 2^24 rows; above, a lone key's planned depth grows by one level
+// per factor of four in rows, from 6 levels at 2^25 to 9 at 2^31, and is
+// deeper with more keys) and partial-row columns for every persistent warp.
 uint64_t key_scratch_bytes(const mg_table* t, int sms) {
   const uint64_t rows = mg_table_rows(t);
-  const uint64_t frontier = (rows <= (1ull << 24) ? rows / 2 : rows >> 8) * 17 + 32 * 17;
+  uint32_t shift = 1;
+  if (rows > (1ull << 24)) {
+    uint32_t lg = 24;
+    while (lg < 32 && (1ull << lg) < rows) ++lg;
+    shift = (lg - 14) / 2;
+  }
+  const uint64_t frontier = (rows >> shift) * 17 + 32 * 17;
   const uint64_t partial = (uint64_t)sms * 4 * 8 * (mg_table_row_bytes(t));
-  return 1200 + frontier + partial;
+  return sizeof(mg::KeyDev) + sizeof(mg::KeyAux) + frontier + partial;
 }
 
 }  // namespace

@@ -1,6 +1,7 @@
-"""GPU parity of the own-rows scan at its launch edges: leaf pairs walked two
+"""GPU parity of the warp kernels at their launch edges: leaf pairs walked two
 at a time (one pair only at depth 1), CTAs from one warp to the full width as
-the items go from fewer than the SMs to several rounds per warp.  Shares are
+the items go from fewer than the SMs to several rounds per warp, and the block
+scan over row sizes, depths and key groups.  Shares are
 exact: the oracle's bytes."""
 import pytest
 
@@ -32,3 +33,49 @@ def test_own_rows_cta_widths(scanner, oracle_mod, row_bytes, M, items):
     assert plan["grid"] <= scanner.device_info()["sm_count"]
     ws.close()
     db.close()
+
+
+@pytest.mark.parametrize("row_bytes", [48, 80, 112, 128, 192, 256, 272, 496, 512])
+@pytest.mark.parametrize("M,keys_per_item,nkeys", [(1, 3, 4), (2, 3, 3), (3, 3, 7), (4, 1, 2), (5, 2, 3), (9, 3, 3)])
+def test_block_scan_shapes(scanner, oracle_mod, row_bytes, M, keys_per_item, nkeys):
+    # Row sizes with every number of rows per warp-wide load from 10 to 1, a
+    # key group left over (fewer keys than the kernel's), a row range that
+    # starts and ends inside a warp tile.
+    d, first, nrows = 18, 12_345, 2 * (32 << M) + 77
+    db = G.GpuPageMatrix.from_seed(scanner, nrows, row_bytes, seed=M, first_row=first)
+    host = oracle_mod.fill_splitmix(first * row_bytes, nrows * row_bytes, M).reshape(nrows, row_bytes)
+    keys = [oracle_keypair(oracle_mod, d, first + (7919 * j) % nrows, seed=91, i=j)[0] for j in range(nkeys)]
+    ws = scanner.workspace()
+    ws.set_shape(M + 5, keys_per_item)
+    ws.set_keys([db] * nkeys, keys)
+    assert ws.plan()["kernel"] == N.KERNEL_WARP
+    want = oracle_mod.scan_fused(keys, host, row_bytes, row_base=first)
+    for graph in (False, True, True):
+        ws.launch(graph=graph)
+        assert ws.read() == want
+    ws.close()
+    db.close()
+
+
+def test_row_sizes_beside_each_other_keep_their_own_keys_per_item(scanner, oracle_mod):
+    # One pass over 32-, 48-, 64- and 256-B tables (and 528 B on the CTA kernel).
+    tabs, keys, want = [], [], []
+    for i, (rb, n) in enumerate([(32, 5000), (48, 3001), (64, 4097), (256, 700), (528, 300)]):
+        host = oracle_mod.fill_splitmix(0, n * rb, 30 + i).reshape(n, rb)
+        t = G.GpuPageMatrix.from_seed(scanner, n, rb, seed=30 + i)
+        for j in range(4):
+            k = oracle_keypair(oracle_mod, 13, (j * 911) % n, seed=92, i=4 * i + j)[0]
+            tabs.append(t)
+            keys.append(k)
+            want += oracle_mod.scan_fused([k], host, rb)
+    assert scanner.scan_multi(list(zip(tabs, keys))) == want
+
+
+def test_pinning_the_warp_kernel_still_needs_a_power_of_two_row(scanner):
+    db = G.GpuPageMatrix.alloc_empty(scanner, 100, 48)
+    key = G.generate_chacha_dpf_keys(G.ChaChaParams(8), 3)[0]
+    ws = scanner.workspace()
+    ws.set_kernel("warp")
+    with pytest.raises(N.MgError):
+        ws.set_keys([db], [key])
+    ws.close()
