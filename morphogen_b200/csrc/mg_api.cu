@@ -854,25 +854,53 @@ int plan_cta(mg_batch* b, const std::vector<SegPlan>& segs, int G, uint32_t col0
   }
 }
 
+// Steps of the frontier chain down to level F, and levels of each but the first.
+constexpr uint32_t kStepLevels = 10;
+uint32_t frontier_steps(uint32_t F) { return F <= kStepLevels ? 1u : (F - 1) / kStepLevels; }
+
+// Levels the CTAs of the chain's first step expand to reach `nodes` nodes of
+// level F (the levels above are walked): the expected fastest.  More levels
+// per CTA mean fewer walks and wider levels, fewer mean more CTAs at work.  3
+// keys, the whole pass: 4099 x 32 B 25.4 us with 6 levels, 32 with 11;
+// 8000000 x 256 B 804 with 11, 825 with 10, 971 with 8.
+uint32_t frontier_levels(uint32_t F, uint64_t nodes, int sms) {
+  constexpr double kLevel = 0.57, kNode = 0.46;  // us: one level's chain; a warp's expansion on a busy scheduler
+  uint32_t best = 0;
+  double best_us = 0;
+  for (uint32_t c = 0; c <= std::min(F, mg::kFrontierLevels); ++c) {
+    const uint32_t wide = std::min(c, mg::kFrontierWide), deep = c - wide, walk = F - c;
+    const double ctas = std::ceil((double)nodes / (double)(1u << c));
+    const double per_sm = std::ceil(ctas / sms);
+    const double warps = std::max(1.0, (double)(1u << wide) / 32.0);
+    const double work = 0.5 * (walk + std::min(wide, 5u)) + (warps - 1.0) + warps * ((1u << deep) - 1.0);
+    const double us = kLevel * (walk + wide) + kNode * ((1u << deep) - 1.0) + per_sm * work * kNode / 4;
+    if (c == 0 || us < best_us) {
+      best_us = us;
+      best = c;
+    }
+  }
+  return best;
+}
+
 // Expected microseconds of a warp-kernel launch that depend on its depth M:
 // the frontier, and the schedulers' rounds of items.  An item is G keys' 2^M - 1
 // node expansions of a warp and V * 2^M row loads per lane; with w of its W
 // warps at work a scheduler runs at the fraction kRate[w] of its full rate.
 // The constants are fitted to passes timed at every M from 1 to 10 (21
 // workloads of 4099 rows to 2^25, 32 to 512 B, 1 to 48 keys): the M it picks is
-// within 3.5% of the fastest in all of them, where the deepest M whose items
+// within 4% of the fastest in all of them and within 5% in 16 others, where the deepest M whose items
 // round up by at most 3% over the schedulers, the rule before, lost up to 54%
 // (300000 x 192 B, 12 keys: 221 us against 144; 100000 x 64 B: 37 against 33).
 double warp_cost_us(uint64_t items, double item_nodes, double item_loads, uint64_t frontier_nodes, int G, bool regroups,
                     uint32_t nw, int sms) {
-  constexpr double kNode = 0.435;         // a warp's node expansion on a busy scheduler
-  constexpr double kLoad = 0.0051;        // a warp-wide row load, and
-  constexpr double kLoadKey = 0.0078;     // its AND/XOR per key
-  constexpr double kItem = 0.22;          // taking an item
-  constexpr double kRegroup = 2.0;        // and changing to another key group's accumulators
-  constexpr double kFrontier = 0.037e-3;  // a frontier node
-  constexpr double kTail = 0.11;          // of an item per warp: warps drift, the last rows are waited for
-  constexpr double kRate[5] = {0.62, 0.72, 0.82, 0.96, 1.0};
+  constexpr double kNode = 0.350;         // a warp's node expansion on a busy scheduler
+  constexpr double kLoad = 0.0095;        // a warp-wide row load, and
+  constexpr double kLoadKey = 0.0087;     // its AND/XOR per key
+  constexpr double kItem = 0.19;          // taking an item
+  constexpr double kRegroup = 1.74;       // and changing to another key group's accumulators
+  constexpr double kFrontier = 0.0495e-3; // a frontier node
+  constexpr double kTail = 0.41;          // of an item per warp: warps drift, the last rows are waited for
+  constexpr double kRate[5] = {0.61, 0.75, 0.95, 0.91, 1.0};
   const uint64_t W = std::max<uint64_t>(1, nw / 4);
   const uint64_t q = (items + (uint64_t)sms * 4 - 1) / ((uint64_t)sms * 4);
   const double item = kNode * item_nodes + item_loads * (kLoad + kLoadKey * G) + kItem + (regroups ? kRegroup : 0.0);
@@ -961,24 +989,23 @@ int plan_warp(mg_batch* b, const std::vector<SegPlan>& segs, int G, uint32_t VT,
       key_bytes[sp.keys[j]] = sp.table->row_bytes;
       key_slot[sp.keys[j]] = (uint32_t)(cursor + j);
     }
-    // Frontier chain: levels 0 -> F = d - M.  Up to kFrontierLevels levels
-    // it is one step from each key's root.  Deeper, every step expands
-    // kFrontierLevels levels below one root per CTA, and the first step's
-    // CTAs reach their roots (level A = F - kFrontierLevels * nsteps, 1..10)
-    // by walking the path from the key's root themselves, so no narrow
-    // one-CTA-per-key step sits above them.
+    // Frontier chain: levels 0 -> F = d - M.  Up to 10 levels it is one step
+    // from each key's root.  Deeper, every further step takes the last 10
+    // levels before it, and the first step's CTAs reach their nodes by walking
+    // the path from the key's root themselves, so no narrow one-CTA-per-key
+    // step sits above them.
     const uint32_t F = sp.d - M;
-    const uint32_t FL = mg::kFrontierLevels;
-    const uint32_t nsteps = F <= FL ? 1u : (F - 1) / FL;
-    const uint32_t A = F <= FL ? 0u : F - FL * nsteps;
+    const uint32_t nsteps = frontier_steps(F);
+    const uint32_t F1 = F - kStepLevels * (nsteps - 1);  // level the first step reaches
+    const uint32_t c1 = frontier_levels(F1, level_count(sp.table, sp.d - F1) * nk, ctx->sms);
+    const uint32_t A = F1 - c1;
     uint32_t Lv = A;
     for (uint32_t st = 0; st < nsteps; ++st) {
       mg::FrontierStep f;
       std::memset(&f, 0, sizeof f);
-      const uint32_t c = F <= FL ? F : FL;
+      const uint32_t c = st == 0 ? c1 : kStepLevels;
       f.L_in = Lv;
       f.c = c;
-      f.per = 1u;
       f.walk = (st == 0 && A > 0) ? 1u : 0u;
       f.n_in = Lv ? level_count(sp.table, sp.d - Lv) : 1;
       f.in_first = Lv ? level_first(sp.table, sp.d - Lv) : 0;
@@ -1225,7 +1252,7 @@ int plan_pass(mg_batch* b) {
     for (uint32_t si = 0; si < L.w.nsegs; ++si) {
       const mg::WarpSeg& sg = L.w.seg[si];
       const uint32_t F = sg.d - sg.M;
-      const uint32_t nsteps = F <= mg::kFrontierLevels ? 1u : (F - 1) / mg::kFrontierLevels;
+      const uint32_t nsteps = frontier_steps(F);
       for (uint32_t k = 0; k < nsteps; ++k, ++st) {
         mg::FrontierStep& f = L.steps[st];
         f.keys = b->d_keys + sg.key_base;

@@ -135,6 +135,44 @@ __device__ __forceinline__ void prg_expand(const uint4 s, uint4& L, uint4& R, ui
   tr = (y[1] + kSigma1) & 1u;
 }
 
+// One of a node expansion's two blocks: L, R hold its words 0-3 and 4-7 (block
+// 0: the children's seeds; block 1: their t bits in bit 0 of L.x and L.y).
+// Two lanes expand a node together where the dependent chain counts and not
+// the throughput: about 1000 cycles, where both blocks in a lane take 1700.
+__device__ __forceinline__ void prg_block(const uint4 s, const uint32_t counter, uint4& L, uint4& R) {
+  uint32_t x[16] = {kSigma0, kSigma1, kSigma2, kSigma3, s.x, s.y, s.z, s.w, s.x, s.y, s.z, s.w, counter, 0u, 0u, 0u};
+  double_round<false, 0>(x);
+  double_round<false, 1>(x);
+  double_round<false, 2>(x);
+  double_round<false, 3>(x);
+  L = make_uint4(x[0] + kSigma0, x[1] + kSigma1, x[2] + kSigma2, x[3] + kSigma3);
+  R = make_uint4(x[4] + s.x, x[5] + s.y, x[6] + s.z, x[7] + s.w);
+}
+
+// The same block over four neighbouring lanes, one column of the state each
+// (all 32 lanes call it): lane `col` of four passes word `col` of the seed and
+// gets words col and 4 + col of the block.  The diagonal rounds cost three
+// shuffles on either side, so the chain is no shorter than prg_block's, but it
+// issues a quarter of the instructions.
+__device__ __forceinline__ void prg_block_quad(const uint32_t col, const uint32_t s, const uint32_t counter, uint32_t& l,
+                                               uint32_t& r) {
+  const uint32_t sigma = col == 0 ? kSigma0 : col == 1 ? kSigma1 : col == 2 ? kSigma2 : kSigma3;
+  uint32_t a = sigma, b = s, c = s, d = col == 0 ? counter : 0u;
+#pragma unroll
+  for (int dr = 0; dr < 4; ++dr) {
+    quarter_round<false, false>(a, b, c, d);
+    b = __shfl_sync(0xFFFFFFFFu, b, (int)(col + 1u) & 3, 4);
+    c = __shfl_sync(0xFFFFFFFFu, c, (int)(col + 2u) & 3, 4);
+    d = __shfl_sync(0xFFFFFFFFu, d, (int)(col + 3u) & 3, 4);
+    quarter_round<false, false>(a, b, c, d);
+    b = __shfl_sync(0xFFFFFFFFu, b, (int)(col + 3u) & 3, 4);
+    c = __shfl_sync(0xFFFFFFFFu, c, (int)(col + 2u) & 3, 4);
+    d = __shfl_sync(0xFFFFFFFFu, d, (int)(col + 1u) & 3, 4);
+  }
+  l = a + sigma;
+  r = b + s;
+}
+
 // One GGM node expansion with the level's correction word applied to both
 // children when t == 1 (dpf.rs:221-239).
 template <bool FMA = true>
@@ -326,16 +364,17 @@ struct WarpScanParams {
   uint32_t queues;      // item queues per CTA: 1, or 4 (one per warp scheduler)
 };
 
-// Levels one frontier-chain step expands (its last level's 2^10 nodes fit the
-// CTA's shared memory).
-constexpr uint32_t kFrontierLevels = 10;
+// Most levels one frontier-chain step expands: breadth first up to
+// kFrontierWide (one node per thread of its CTA), the rest depth first.
+constexpr uint32_t kFrontierWide = 8;
+constexpr uint32_t kFrontierLevels = 11;
 
-// One breadth-first step of the frontier chain: every CTA expands `per`
-// nodes of level L_in of key blockIdx.y by c <= kFrontierLevels levels and
-// stores the nodes of level L_in + c that meet the table.  With `walk` set
-// (per == 1) the CTA's root is not read from in_seed: the CTA derives it from
-// the key's root by the L_in-level path walk of ChaCha::eval, so the first
-// step of a chain needs no narrow one-CTA-per-key launch above it.
+// One step of the frontier chain: every CTA expands one node of
+// level L_in of key blockIdx.y by c <= kFrontierLevels levels and stores the
+// nodes of level L_in + c that meet the table.  With `walk` set the CTA's root
+// is not read from in_seed: the CTA derives it from the key's root by the
+// L_in-level path walk of ChaCha::eval, so the first step of a chain needs no
+// narrow one-CTA-per-key launch above it.
 struct FrontierStep {
   const KeyDev* keys;     // the segment's keys
   const uint4* in_seed;   // level L_in (unused when L_in == 0): key j at j * n_in
@@ -350,7 +389,6 @@ struct FrontierStep {
   uint64_t out_stride;
   uint32_t L_in;
   uint32_t c;
-  uint32_t per;           // input nodes per CTA (per << c <= 2^kFrontierLevels)
   uint32_t walk;          // 1: each CTA walks from the key's root to its level-L_in node
   uint4* zero_out;        // CTA (0, 0) zeroes these zero_n shares first (or null)
   uint64_t zero_n;

@@ -245,92 +245,163 @@ __global__ void __launch_bounds__(kThreads, (G <= 4 ? 3 : 2)) scan_kernel(const 
 
 // ---- warp-independent path -------------------------------------------------
 
-// Frontier chain step: CTA (x, key) expands the `per` consecutive input slots
-// x * per .. (level indices in_first + slot) of level L_in of key `blockIdx.y`
-// by c <= kFrontierLevels levels breadth-first in shared memory (per * 2^c <=
-// 2^kFrontierLevels nodes) and stores the nodes of level L_in + c that
-// intersect the table, at slot (level index - out_first).  Several roots per
-// CTA keep the top levels of a wide step busy; the first step (one root per
-// key) is a latency chain either way.  The c levels' correction words are
-// loaded into shared memory once, up front, so the level-by-level expansion
-// waits on no memory access.
+// Frontier chain step: CTA (x, key) takes node x of level L_in (level index
+// in_first + x) of key `blockIdx.y` c levels down and stores the nodes of level
+// L_in + c that intersect the table, at slot (level index - out_first).
+//
+// The levels are a serial chain, so what bounds a small frontier is the time of
+// one node expansion (0.57 us a level), and a large one the share of full warps
+// (26 G nodes/s: ALU pipe 81% busy at 3 x 2^20 nodes, 118 us; 151 us with every
+// level breadth first and one lane per node).  The path to the CTA's node (with
+// walk) and the first min(c, 8) levels below it go breadth first in shared
+// memory: up to 4 nodes with eight lanes per node, up to 128 with two, the even
+// one computing block 0 (both children's seeds), the odd one block 1 (their t
+// bits).  Levels of up to 16 nodes run in warp 0 without a CTA barrier.  The
+// last c - 8 levels are walked depth first, one of the 256 nodes per thread,
+// with no barrier at all.
 __global__ void __launch_bounds__(kThreads) frontier_kernel(const __grid_constant__ FrontierStep f) {
-  constexpr uint32_t kNodes = 1u << kFrontierLevels;
-  __shared__ uint4 sa[kNodes], sb[kNodes];
-  __shared__ uint8_t ta[kNodes], tb[kNodes];
-  __shared__ uint4 s_cw[kFrontierLevels];
-  __shared__ uint32_t s_cwl[kFrontierLevels], s_cwr[kFrontierLevels];
-  const uint32_t tid = threadIdx.x;
-  const uint64_t node0 = (uint64_t)blockIdx.x * f.per, j = blockIdx.y;
+  constexpr uint32_t kWide = 1u << kFrontierWide;  // nodes of the widest breadth-first level
+  static_assert(kWide == kThreads, "one node per thread for the depth-first levels");
+  __shared__ uint4 sa[kWide], sb[kWide];
+  __shared__ uint8_t ta[kWide], tb[kWide];
+  __shared__ uint4 stk[kFrontierLevels - kFrontierWide - 1][kWide];
+  __shared__ uint8_t stk_t[kFrontierLevels - kFrontierWide - 1][kWide];
+  __shared__ uint4 s_cw[kMaxLevels];
+  __shared__ uint32_t s_cwt[2][kMaxLevels];  // t correction bytes: left, right
+  const uint32_t tid = threadIdx.x, half = tid & 1u;
+  const uint64_t node = blockIdx.x, j = blockIdx.y;
   // The pass's shares start at zero: the scan CTAs XOR into them.
   if (f.zero_out && blockIdx.x == 0 && blockIdx.y == 0)
     for (uint64_t i = tid; i < f.zero_n; i += kThreads) f.zero_out[i] = make_uint4(0u, 0u, 0u, 0u);
-  const uint32_t nroots = (uint32_t)(f.n_in - node0 < f.per ? f.n_in - node0 : f.per);
-  const uint64_t g_out0 = (f.in_first + node0) << f.c;  // level index of the first child
-  const uint64_t n = (uint64_t)nroots << f.c;
-  if (g_out0 + n <= f.out_first || g_out0 >= f.out_first + f.n_out) return;  // uniform per CTA
+  const uint64_t a = f.in_first + node;  // level index of the CTA's node
+  const uint64_t g_out0 = a << f.c;      // level index of its first descendant
+  if (g_out0 + (1ull << f.c) <= f.out_first || g_out0 >= f.out_first + f.n_out) return;  // uniform per CTA
   const KeyDev* __restrict__ K = f.keys + j;
-  if (tid < f.c) {
-    s_cw[tid] = __ldg(&K->cw_seed[f.L_in + tid]);
-    s_cwl[tid] = __ldg(&K->cw_tl[f.L_in + tid]);
-    s_cwr[tid] = __ldg(&K->cw_tr[f.L_in + tid]);
-  }
-  if (f.L_in == 0 || f.walk) {
-    // The CTA's root (per == 1 when walking): node in_first + node0 of level
-    // L_in, reached from the key's root as ChaCha::eval does (dpf.rs:103-142).
-    // Warp 1 walks while warp 0 loads the step's correction words.
-    if ((tid >> 5) == 1) {
-      uint4 s = __ldg(&K->root_seed);
-      uint32_t t = __ldg(&K->root_t);
-      const uint64_t a = f.in_first + node0;
-      for (uint32_t lvl = 0; lvl < f.L_in; ++lvl) {
-        uint4 Lc, Rc;
-        uint32_t tl, tr;
-        expand_cw_g<false>(s, t, K, lvl, Lc, tl, Rc, tr);
-        const uint32_t bit = (uint32_t)(a >> (f.L_in - 1 - lvl)) & 1u;
-        s = bit ? Rc : Lc;
-        t = bit ? tr : tl;
-      }
-      if (tid == 32) {
-        sa[0] = s;
-        ta[0] = (uint8_t)t;
-      }
+  const uint32_t walk = f.walk ? f.L_in : 0u;  // levels above the CTA's node
+  const uint32_t top = f.L_in - walk;          // level of the first node expanded
+  const uint32_t wide = f.c < kFrontierWide ? f.c : kFrontierWide;
+  const uint32_t deep = f.c - wide;
+  if (tid < kMaxLevels) {
+    // Correction words of the step's levels, and its root.
+    const uint32_t lvl = top + tid;
+    if (tid < walk + f.c) {
+      s_cw[tid] = __ldg(&K->cw_seed[lvl]);
+      s_cwt[0][tid] = __ldg(&K->cw_tl[lvl]);
+      s_cwt[1][tid] = __ldg(&K->cw_tr[lvl]);
     }
-  } else {
-    for (uint32_t r = tid; r < nroots; r += kThreads) {
-      sa[r] = f.in_seed[j * f.n_in + node0 + r];
-      ta[r] = f.in_t[j * f.n_in + node0 + r];
+    if (tid == 0) {
+      sa[0] = top == 0 ? __ldg(&K->root_seed) : f.in_seed[j * f.n_in + node];
+      ta[0] = (uint8_t)(top == 0 ? __ldg(&K->root_t) : f.in_t[j * f.n_in + node]);
     }
   }
-  __syncthreads();
   uint4* cs = sa; uint8_t* ct = ta;
   uint4* ns = sb; uint8_t* nt = tb;
-  for (uint32_t lv = 0; lv < f.c; ++lv) {
-    // Level lv holds nroots * 2^lv nodes, root-major; node i's children are
-    // 2i and 2i + 1 of the next level.
-    for (uint32_t i = tid; i < (nroots << lv); i += kThreads) {
-      uint4 Lc, Rc;
-      uint32_t tl, tr;
-      prg_expand(cs[i], Lc, Rc, tl, tr);
-      // dpf.rs:221-239: correction word on both children when t == 1.
-      const uint32_t m = (ct[i] == 1) ? 0xFFFFFFFFu : 0u;
-      const uint4 cw = s_cw[lv];
-      Lc.x ^= cw.x & m; Lc.y ^= cw.y & m; Lc.z ^= cw.z & m; Lc.w ^= cw.w & m;
-      Rc.x ^= cw.x & m; Rc.y ^= cw.y & m; Rc.z ^= cw.z & m; Rc.w ^= cw.w & m;
-      ns[2 * i] = Lc;
-      ns[2 * i + 1] = Rc;
-      nt[2 * i] = (uint8_t)(tl ^ (s_cwl[lv] & m));
-      nt[2 * i + 1] = (uint8_t)(tr ^ (s_cwr[lv] & m));
-    }
-    __syncthreads();
+  auto swap = [&]() {
     uint4* x = cs; cs = ns; ns = x;
     uint8_t* y = ct; ct = nt; nt = y;
+  };
+  // Levels of at most 4 nodes: eight lanes of warp 0 per node (block, column).
+  const uint32_t tiny = walk + (wide < 3u ? wide : 3u);
+  if (tid < 32) {
+    const uint32_t i = tid >> 3, blk = (tid >> 2) & 1u, col = tid & 3u;
+#pragma unroll 1
+    for (uint32_t lv = 0; lv < tiny; ++lv) {
+      __syncwarp();
+      const uint32_t n = lv < walk ? 1u : 1u << (lv - walk);  // nodes of the level
+      const uint32_t s = reinterpret_cast<const uint32_t*>(cs)[(i < n ? 4 * i : 0u) + col];
+      // dpf.rs:221-239: correction word on both children when t == 1.
+      const uint32_t m = ct[i < n ? i : 0u] == 1 ? 0xFFFFFFFFu : 0u;
+      uint32_t l, r;
+      prg_block_quad(col, s, blk, l, r);
+      if (i < n) {
+        // On the path (dpf.rs:103-142) only the child towards node a is kept.
+        const bool path = lv < walk;
+        const uint32_t bit = path ? (uint32_t)(a >> (walk - 1 - lv)) & 1u : 0u;
+        if (blk == 0) {
+          const uint32_t cw = reinterpret_cast<const uint32_t*>(s_cw)[4 * lv + col] & m;
+          uint32_t* const dst = reinterpret_cast<uint32_t*>(ns) + (path ? 0u : 8 * i) + col;
+          dst[0] = (bit ? r : l) ^ cw;
+          if (!path) dst[4] = r ^ cw;
+        } else if (col < 2 && (!path || col == bit)) {
+          nt[path ? 0u : 2 * i + col] = (uint8_t)((l & 1u) ^ (s_cwt[col][lv] & m));
+        }
+      }
+      swap();
+    }
+  } else if (tiny & 1u) {
+    swap();
   }
-  for (uint32_t i = tid; i < n; i += kThreads) {
-    const uint64_t o = g_out0 + i - f.out_first;  // wraps for children before the range
+  // Levels of 8 to 128 nodes: two lanes per node, those of warp 0 without a
+  // CTA barrier.
+#pragma unroll 1
+  for (uint32_t lv = tiny; lv < walk + wide; ++lv) {
+    const uint32_t n = 1u << (lv - walk);
+    if (n > 16)
+      __syncthreads();
+    else if (tid < 32)
+      __syncwarp();
+    if (tid < 2 * n) {
+      const uint32_t i = tid >> 1;
+      const uint32_t m = ct[i] == 1 ? 0xFFFFFFFFu : 0u;
+      uint4 L, R;
+      prg_block(cs[i], half, L, R);
+      if (half == 0) {
+        const uint4 cw = s_cw[lv];
+        ns[2 * i] = make_uint4(L.x ^ (cw.x & m), L.y ^ (cw.y & m), L.z ^ (cw.z & m), L.w ^ (cw.w & m));
+        ns[2 * i + 1] = make_uint4(R.x ^ (cw.x & m), R.y ^ (cw.y & m), R.z ^ (cw.z & m), R.w ^ (cw.w & m));
+      } else {
+        nt[2 * i] = (uint8_t)((L.x & 1u) ^ (s_cwt[0][lv] & m));
+        nt[2 * i + 1] = (uint8_t)((L.y & 1u) ^ (s_cwt[1][lv] & m));
+      }
+    }
+    swap();
+  }
+  __syncthreads();
+  if (tid >= (1u << wide)) return;
+  // Thread tid's node and its 2^deep descendants.
+  uint4* const out_seed = f.out_seed + f.out_base + j * f.out_stride;
+  uint8_t* const out_t = f.out_t + f.out_base + j * f.out_stride;
+  auto store = [&](uint32_t i, const uint4 s, uint32_t t) {
+    const uint64_t o = g_out0 + i - f.out_first;  // wraps for nodes before the range
     if (o < f.n_out) {
-      f.out_seed[f.out_base + j * f.out_stride + o] = cs[i];
-      f.out_t[f.out_base + j * f.out_stride + o] = ct[i];
+      out_seed[o] = s;
+      out_t[o] = (uint8_t)t;
+    }
+  };
+  uint4 s = cs[tid];
+  uint32_t t = ct[tid];
+  if (deep == 0) {
+    store(tid, s, t);
+    return;
+  }
+#pragma unroll 1
+  for (uint32_t pi = 0; pi < (1u << (deep - 1)); ++pi) {
+    uint32_t lvl = 0;
+    if (pi) {
+      lvl = deep - (uint32_t)__ffs((int)pi);
+      s = stk[lvl - 1][tid];
+      t = stk_t[lvl - 1][tid];
+    }
+    for (;; ++lvl) {
+      uint4 L, R;
+      uint32_t tl, tr;
+      prg_expand(s, L, R, tl, tr);
+      const uint32_t m = t == 1u ? 0xFFFFFFFFu : 0u;
+      const uint4 cw = s_cw[walk + wide + lvl];
+      L.x ^= cw.x & m; L.y ^= cw.y & m; L.z ^= cw.z & m; L.w ^= cw.w & m;
+      R.x ^= cw.x & m; R.y ^= cw.y & m; R.z ^= cw.z & m; R.w ^= cw.w & m;
+      tl ^= s_cwt[0][walk + wide + lvl] & m;
+      tr ^= s_cwt[1][walk + wide + lvl] & m;
+      if (lvl + 1 == deep) {
+        const uint32_t i = (tid << deep) + 2 * pi;
+        store(i, L, tl);
+        store(i + 1, R, tr);
+        break;
+      }
+      stk[lvl][tid] = R;
+      stk_t[lvl][tid] = (uint8_t)tr;
+      s = L;
+      t = tl;
     }
   }
 }
@@ -1233,9 +1304,8 @@ cudaError_t launch_delta(const KeyDev* keys, const uint2* jobs, uint32_t njobs, 
 
 cudaError_t launch_frontier(const FrontierStep& f, uint32_t nkeys, cudaStream_t st) {
   if (f.n_in == 0 || nkeys == 0) return cudaSuccess;
-  if (f.per == 0 || ((uint64_t)f.per << f.c) > (1ull << kFrontierLevels)) return cudaErrorInvalidValue;
-  if (f.walk && (f.per != 1 || f.L_in >= (uint32_t)kMaxLevels)) return cudaErrorInvalidValue;
-  dim3 grid((unsigned)((f.n_in + f.per - 1) / f.per), nkeys);
+  if (f.c > kFrontierLevels || f.L_in + f.c > (uint32_t)kMaxLevels) return cudaErrorInvalidValue;
+  dim3 grid((unsigned)f.n_in, nkeys);
   frontier_kernel<<<grid, kThreads, 0, st>>>(f);
   return cudaGetLastError();
 }

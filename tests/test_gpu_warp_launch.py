@@ -79,3 +79,30 @@ def test_pinning_the_warp_kernel_still_needs_a_power_of_two_row(scanner):
     with pytest.raises(N.MgError):
         ws.set_keys([db], [key])
     ws.close()
+
+
+@pytest.mark.parametrize("d,M,first,nrows", [
+    (23, 1, 5, 4_194_304),          # 11 levels per CTA, the last three depth first
+    (20, 3, 0, 1_000_000),          # 10 or 11
+    (26, 4, 1 << 25, 300_001),      # walk from the root to a range in the middle
+    (9, 1, 0, 512), (9, 8, 0, 512), (9, 9, 0, 512),  # 8, 1 and 0 frontier levels
+    (32, 1, (1 << 32) - 3001, 3001),
+])
+def test_frontier_levels_per_cta(scanner, oracle_mod, d, M, first, nrows):
+    # The levels a frontier CTA expands (and so its walk) follow the number of
+    # nodes; keys with non-binary t correction bytes take the same path.
+    db = G.GpuPageMatrix.from_seed(scanner, nrows, 16, seed=d, first_row=first)
+    host = oracle_mod.fill_splitmix(first * 16, nrows * 16, d).reshape(nrows, 16)
+    keys = [oracle_keypair(oracle_mod, d, first + (12_347 * j) % nrows, seed=93, i=j)[0] for j in range(2)]
+    odd = bytearray(keys[1])
+    for lvl in range(0, d, 3):
+        odd[19 + 18 * lvl + 16] ^= 2  # left t byte 2 or 3
+    keys.append(bytes(odd))
+    ws = scanner.workspace()
+    ws.set_kernel("warp")
+    ws.set_shape(M + 5, 1)
+    ws.set_keys([db] * 3, keys)
+    ws.launch()
+    assert ws.read() == oracle_mod.scan_fused(keys, host, 16, row_base=first)
+    ws.close()
+    db.close()
