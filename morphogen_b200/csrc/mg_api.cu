@@ -197,6 +197,7 @@ struct mg_batch {
     uint32_t cols = 0;
     size_t smem = 0;
     int G = 1;
+    bool fma = false;      // CTA kernel: PRG form
     uint32_t VT = 0;
     uint32_t NW = 0;       // warp kernel: warps per CTA
     uint32_t col0 = 0;     // first share column of this launch
@@ -280,9 +281,9 @@ int set_device(const T* obj) {
 // The kernels' shared-memory limits are process-wide per device; the
 // launchers keep one high-water mark for every caller (scan_prepare /
 // warp_prepare only raise it), so nothing is cached per context.
-int prepare_g(mg_context* ctx, int G, size_t smem) {
+int prepare_g(mg_context* ctx, int G, bool fma, size_t smem) {
   (void)ctx;
-  MG_CUDA(mg::scan_prepare(G, smem));
+  MG_CUDA(mg::scan_prepare(G, fma, smem));
   return MG_OK;
 }
 
@@ -785,75 +786,6 @@ int mg_batch_set_kernel(mg_batch* b, int kind) {
 
 namespace {
 
-// Plan one CTA-kernel launch over segs (at most kMaxSegs): tile depth S, the
-// deepest in [8, 14] that still gives >= 4 waves of items (or the pinned one).
-int plan_cta(mg_batch* b, const std::vector<SegPlan>& segs, int G, uint32_t col0, size_t& key_cursor,
-             std::vector<uint32_t>& key_col, std::vector<uint32_t>& key_bytes, std::vector<uint32_t>& key_slot,
-             mg_batch::Launch& out) {
-  mg_context* ctx = b->ctx;
-  for (uint32_t S_target = b->eff_S ? b->eff_S : 14;; --S_target) {
-    mg_batch::Launch L;
-    std::memset(&L.p, 0, sizeof L.p);
-    L.kind = MG_KERNEL_CTA;
-    L.G = G;
-    L.col0 = col0;
-    uint32_t slots = 2, cols = 0;
-    uint64_t items = 0;
-    size_t cursor = key_cursor;
-    std::vector<std::pair<uint32_t, uint32_t>> assign;  // (key, column)
-    for (size_t si = 0; si < segs.size(); ++si) {
-      const SegPlan& sp = segs[si];
-      mg::Segment& sg = L.p.seg[si];
-      uint32_t S, U, M;
-      shape_for(sp.d, S_target, S, U, M);
-      sg.table = reinterpret_cast<const uint4*>(sp.table->d);
-      sg.first = sp.table->first;
-      sg.rows = sp.table->rows;
-      sg.V = sp.table->row_bytes / 16;
-      sg.d = sp.d;
-      sg.S = S;
-      sg.U = U;
-      sg.M = M;
-      sg.g = sp.g;
-      sg.groups = (uint32_t)(sp.keys.size() / sp.g);
-      sg.tiles = (uint32_t)level_count(sp.table, S);
-      sg.item_begin = items;
-      sg.key_base = (uint32_t)cursor;
-      sg.col_base = cols;
-      for (size_t j = 0; j < sp.keys.size(); ++j) {
-        key_col[sp.keys[j]] = col0 + cols + (uint32_t)j * sg.V;
-        key_bytes[sp.keys[j]] = sp.table->row_bytes;
-        key_slot[sp.keys[j]] = (uint32_t)(cursor + j);
-      }
-      cursor += sp.keys.size();
-      items += (uint64_t)sg.tiles * sg.groups;
-      cols += (uint32_t)sp.keys.size() * sg.V;
-      slots = std::max(slots, M);
-    }
-    L.p.nsegs = (uint32_t)segs.size();
-    L.p.items = items;
-    L.p.cols = cols;
-    L.p.slots = slots;
-    L.cols = cols;
-    L.smem = mg::scan_smem_bytes(G, slots);
-    int occ = 0;
-    if (L.smem <= ctx->smem_optin) {
-      if (int rc = prepare_g(ctx, G, L.smem)) return rc;
-      occ = mg::scan_occupancy(G, L.smem);
-    }
-    const uint64_t slots_total = (uint64_t)std::max(occ, 1) * ctx->sms;
-    const bool enough = occ > 0 && items >= 4 * slots_total;
-    if (b->eff_S || enough || S_target <= 8) {
-      if (occ <= 0) return fail(MG_EINVAL, "launch shape S=%u G=%d does not fit the device", S_target, G);
-      L.grid = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(items, slots_total));
-      L.nparts = L.grid;
-      key_cursor = cursor;
-      out = std::move(L);
-      return MG_OK;
-    }
-  }
-}
-
 // Steps of the frontier chain down to level F, and levels of each but the first.
 constexpr uint32_t kStepLevels = 10;
 uint32_t frontier_steps(uint32_t F) { return F <= kStepLevels ? 1u : (F - 1) / kStepLevels; }
@@ -880,6 +812,140 @@ uint32_t frontier_levels(uint32_t F, uint64_t nodes, int sms) {
     }
   }
   return best;
+}
+
+// Append the frontier chain of a segment to its launch: for every key the nodes
+// of level F whose subtrees meet the table, at frontier index fr_base.  Up to 10
+// levels it is one step from each key's root.  Deeper, every further step takes
+// the last 10 levels before it, and the first step's CTAs reach their nodes by
+// walking the path from the key's root themselves, so no narrow
+// one-CTA-per-key step sits above them.
+void add_frontier(mg_batch::Launch& L, const SegPlan& sp, uint32_t F, uint64_t fr_base, size_t& tmp_need, int sms) {
+  const uint32_t nk = (uint32_t)sp.keys.size();
+  const uint32_t nsteps = frontier_steps(F);
+  const uint32_t F1 = F - kStepLevels * (nsteps - 1);  // level the first step reaches
+  const uint32_t c1 = frontier_levels(F1, level_count(sp.table, sp.d - F1) * nk, sms);
+  uint32_t Lv = F1 - c1;
+  for (uint32_t st = 0; st < nsteps; ++st) {
+    mg::FrontierStep f;
+    std::memset(&f, 0, sizeof f);
+    const uint32_t c = st == 0 ? c1 : kStepLevels;
+    f.L_in = Lv;
+    f.c = c;
+    f.walk = (st == 0 && Lv > 0) ? 1u : 0u;
+    f.n_in = Lv ? level_count(sp.table, sp.d - Lv) : 1;
+    f.in_first = Lv ? level_first(sp.table, sp.d - Lv) : 0;
+    f.n_out = level_count(sp.table, sp.d - (Lv + c));
+    f.out_first = level_first(sp.table, sp.d - (Lv + c));
+    const bool last = st + 1 == nsteps;
+    f.out_base = last ? fr_base : 0;
+    f.out_stride = f.n_out;
+    if (!last) tmp_need = std::max<size_t>(tmp_need, (size_t)nk * f.n_out);
+    L.steps.push_back(f);  // pointers are set once the workspace has its buffers
+    L.step_keys.push_back(nk);
+    Lv += c;
+  }
+}
+
+// Set the pointers of one segment's chain, L.steps[st..]; returns the index
+// behind it.
+size_t wire_frontier(mg_batch* b, mg_batch::Launch& L, size_t st, uint32_t F, uint32_t key_base) {
+  const uint32_t nsteps = frontier_steps(F);
+  for (uint32_t k = 0; k < nsteps; ++k, ++st) {
+    mg::FrontierStep& f = L.steps[st];
+    f.keys = b->d_keys + key_base;
+    f.in_seed = k ? b->d_tmp_seed[(k - 1) & 1] : nullptr;
+    f.in_t = k ? b->d_tmp_t[(k - 1) & 1] : nullptr;
+    const bool last = k + 1 == nsteps;
+    f.out_seed = last ? b->d_fr_seed : b->d_tmp_seed[k & 1];
+    f.out_t = last ? b->d_fr_t : b->d_tmp_t[k & 1];
+  }
+  return st;
+}
+
+// Plan one CTA-kernel launch over segs (at most kMaxSegs): tile depth S, the
+// deepest in [8, 14] that still gives >= 4 waves of items (or the pinned one).
+int plan_cta(mg_batch* b, const std::vector<SegPlan>& segs, int G, uint32_t col0, size_t& key_cursor,
+             std::vector<uint32_t>& key_col, std::vector<uint32_t>& key_bytes, std::vector<uint32_t>& key_slot,
+             uint64_t& fr_cursor, size_t& tmp_need, mg_batch::Launch& out) {
+  mg_context* ctx = b->ctx;
+  for (uint32_t S_target = b->eff_S ? b->eff_S : 14;; --S_target) {
+    mg_batch::Launch L;
+    std::memset(&L.p, 0, sizeof L.p);
+    L.kind = MG_KERNEL_CTA;
+    L.G = G;
+    L.col0 = col0;
+    uint32_t slots = 2, cols = 0, Vmax = 1;
+    uint64_t items = 0;
+    size_t cursor = key_cursor, tmp = tmp_need;
+    uint64_t fr = fr_cursor;
+    for (size_t si = 0; si < segs.size(); ++si) {
+      const SegPlan& sp = segs[si];
+      mg::Segment& sg = L.p.seg[si];
+      uint32_t S, U, M;
+      shape_for(sp.d, S_target, S, U, M);
+      sg.table = reinterpret_cast<const uint4*>(sp.table->d);
+      sg.first = sp.table->first;
+      sg.rows = sp.table->rows;
+      sg.V = sp.table->row_bytes / 16;
+      sg.d = sp.d;
+      sg.S = S;
+      sg.U = U;
+      sg.M = M;
+      sg.g = sp.g;
+      sg.groups = (uint32_t)(sp.keys.size() / sp.g);
+      sg.tiles = (uint32_t)level_count(sp.table, S);
+      sg.item_begin = items;
+      sg.key_base = (uint32_t)cursor;
+      sg.col_base = cols;
+      for (size_t j = 0; j < sp.keys.size(); ++j) {
+        key_col[sp.keys[j]] = col0 + cols + (uint32_t)j * sg.V;
+        key_bytes[sp.keys[j]] = sp.table->row_bytes;
+        key_slot[sp.keys[j]] = (uint32_t)(cursor + j);
+      }
+      sg.fr_base = fr;
+      add_frontier(L, sp, sp.d - S, fr, tmp, ctx->sms);
+      fr += (uint64_t)sg.tiles * sp.keys.size();
+      Vmax = std::max(Vmax, sg.V);
+      cursor += sp.keys.size();
+      items += (uint64_t)sg.tiles * sg.groups;
+      cols += (uint32_t)sp.keys.size() * sg.V;
+      slots = std::max(slots, M);
+    }
+    L.p.nsegs = (uint32_t)segs.size();
+    L.p.items = items;
+    L.p.cols = cols;
+    L.p.slots = slots;
+    L.cols = cols;
+    L.smem = mg::scan_smem_bytes(G, slots);
+    L.fma = mg::scan_fma(Vmax);
+    int occ = 0;
+    if (L.smem <= ctx->smem_optin) {
+      if (int rc = prepare_g(ctx, G, L.fma, L.smem)) return rc;
+      occ = mg::scan_occupancy(G, L.fma, L.smem);
+    }
+    const uint64_t slots_total = (uint64_t)std::max(occ, 1) * ctx->sms;
+    const bool enough = occ > 0 && items >= 4 * slots_total;
+    if (b->eff_S || enough || S_target <= 8) {
+      if (occ <= 0) return fail(MG_EINVAL, "launch shape S=%u G=%d does not fit the device", S_target, G);
+      L.grid = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(items, slots_total));
+      L.nparts = L.grid;
+      key_cursor = cursor;
+      // CTAs that take several items read their tiles' roots from a frontier;
+      // with one item each, the walk inside the kernel is shorter than another
+      // launch (3 keys, 3000 x 4 KB: 57 us against 64; 200000 x 4 KB, 1.8 items
+      // per CTA: 191 against 186; 500000 x 1 KB: 189 against 166).
+      if (items > L.grid) {
+        fr_cursor = fr;
+        tmp_need = tmp;
+      } else {
+        L.steps.clear();
+        L.step_keys.clear();
+      }
+      out = std::move(L);
+      return MG_OK;
+    }
+  }
 }
 
 // Expected microseconds of a warp-kernel launch that depend on its depth M:
@@ -989,37 +1055,7 @@ int plan_warp(mg_batch* b, const std::vector<SegPlan>& segs, int G, uint32_t VT,
       key_bytes[sp.keys[j]] = sp.table->row_bytes;
       key_slot[sp.keys[j]] = (uint32_t)(cursor + j);
     }
-    // Frontier chain: levels 0 -> F = d - M.  Up to 10 levels it is one step
-    // from each key's root.  Deeper, every further step takes the last 10
-    // levels before it, and the first step's CTAs reach their nodes by walking
-    // the path from the key's root themselves, so no narrow one-CTA-per-key
-    // step sits above them.
-    const uint32_t F = sp.d - M;
-    const uint32_t nsteps = frontier_steps(F);
-    const uint32_t F1 = F - kStepLevels * (nsteps - 1);  // level the first step reaches
-    const uint32_t c1 = frontier_levels(F1, level_count(sp.table, sp.d - F1) * nk, ctx->sms);
-    const uint32_t A = F1 - c1;
-    uint32_t Lv = A;
-    for (uint32_t st = 0; st < nsteps; ++st) {
-      mg::FrontierStep f;
-      std::memset(&f, 0, sizeof f);
-      const uint32_t c = st == 0 ? c1 : kStepLevels;
-      f.L_in = Lv;
-      f.c = c;
-      f.walk = (st == 0 && A > 0) ? 1u : 0u;
-      f.n_in = Lv ? level_count(sp.table, sp.d - Lv) : 1;
-      f.in_first = Lv ? level_first(sp.table, sp.d - Lv) : 0;
-      f.n_out = level_count(sp.table, sp.d - (Lv + c));
-      f.out_first = level_first(sp.table, sp.d - (Lv + c));
-      const bool last = st + 1 == nsteps;
-      f.out_base = last ? fr_cursor : 0;
-      f.out_stride = last ? nF : f.n_out;
-      if (!last) tmp_need = std::max<size_t>(tmp_need, (size_t)nk * f.n_out);
-      f.keys = nullptr;  // set after allocation (key_base offset kept in in_t slot below)
-      L.steps.push_back(f);
-      L.step_keys.push_back(nk);
-      Lv += c;
-    }
+    add_frontier(L, sp, sp.d - M, fr_cursor, tmp_need, ctx->sms);
     fr_cursor += (uint64_t)nk * nF;
     cursor += nk;
     items += (uint64_t)sg.groups * sg.tiles;
@@ -1065,7 +1101,8 @@ static int enqueue_pass(mg_batch* b, cudaStream_t st, cudaEvent_t mark, bool out
   for (size_t i = 0; i < b->launches.size(); ++i) {
     const mg_batch::Launch& L = b->launches[i];
     if (L.kind == MG_KERNEL_CTA) {
-      MG_CUDA(mg::launch_scan(L.G, L.p, L.grid, L.smem, st));
+      for (size_t k = 0; k < L.steps.size(); ++k) MG_CUDA(mg::launch_frontier(L.steps[k], L.step_keys[k], st));
+      MG_CUDA(mg::launch_scan(L.G, L.fma, L.p, L.grid, L.smem, st));
     } else if (!mg::warp_reduces_in_kernel(L.G, L.VT)) {
       for (size_t k = 0; k < L.steps.size(); ++k) MG_CUDA(mg::launch_frontier(L.steps[k], L.step_keys[k], st));
       MG_CUDA(mg::launch_scan_warp(L.G, L.VT, L.w, L.grid, L.NW, L.smem, st));
@@ -1169,7 +1206,7 @@ int plan_pass(mg_batch* b) {
     std::vector<SegPlan> chunk(cta_segs.begin() + s0,
                                cta_segs.begin() + std::min(cta_segs.size(), s0 + mg::kMaxSegs));
     mg_batch::Launch L;
-    if (int rc = plan_cta(b, chunk, Gc, total_cols, key_cursor, key_col, key_bytes, key_slot, L)) return rc;
+    if (int rc = plan_cta(b, chunk, Gc, total_cols, key_cursor, key_col, key_bytes, key_slot, fr_cursor, tmp_need, L)) return rc;
     total_cols += L.cols;
     launches.push_back(std::move(L));
   }
@@ -1236,9 +1273,15 @@ int plan_pass(mg_batch* b) {
     make_aux(parsed[i], &h_aux[key_slot[i]]);
   }
   for (mg_batch::Launch& L : launches) {
+    size_t st = 0;
     if (L.kind == MG_KERNEL_CTA) {
       L.p.keys = b->d_keys;
       L.p.partial = b->d_partial;
+      if (L.steps.empty()) continue;
+      L.p.fr_seed = b->d_fr_seed;
+      L.p.fr_t = b->d_fr_t;
+      for (uint32_t si = 0; si < L.p.nsegs; ++si)
+        st = wire_frontier(b, L, st, L.p.seg[si].d - L.p.seg[si].S, L.p.seg[si].key_base);
       continue;
     }
     L.w.keys = b->d_keys;
@@ -1247,22 +1290,8 @@ int plan_pass(mg_batch* b) {
     L.w.fr_t = b->d_fr_t;
     L.w.partial = b->d_partial;
     L.w.out = b->d_out + L.col0;
-    // Wire the frontier chains: each segment's steps are consecutive.
-    size_t st = 0;
-    for (uint32_t si = 0; si < L.w.nsegs; ++si) {
-      const mg::WarpSeg& sg = L.w.seg[si];
-      const uint32_t F = sg.d - sg.M;
-      const uint32_t nsteps = frontier_steps(F);
-      for (uint32_t k = 0; k < nsteps; ++k, ++st) {
-        mg::FrontierStep& f = L.steps[st];
-        f.keys = b->d_keys + sg.key_base;
-        f.in_seed = k ? b->d_tmp_seed[(k - 1) & 1] : nullptr;
-        f.in_t = k ? b->d_tmp_t[(k - 1) & 1] : nullptr;
-        const bool last = k + 1 == nsteps;
-        f.out_seed = last ? b->d_fr_seed : b->d_tmp_seed[k & 1];
-        f.out_t = last ? b->d_fr_t : b->d_tmp_t[k & 1];
-      }
-    }
+    for (uint32_t si = 0; si < L.w.nsegs; ++si)
+      st = wire_frontier(b, L, st, L.w.seg[si].d - L.w.seg[si].M, L.w.seg[si].key_base);
   }
   MG_CUDA(cudaMemcpyAsync(b->d_keys, b->h_keys, (size_t)nkeys * (sizeof(KeyDev) + sizeof(mg::KeyAux)),
                           cudaMemcpyHostToDevice, b->stream));
@@ -1563,6 +1592,7 @@ std::vector<uint8_t> pass_signature(const mg_batch* b) {
     add(&L.grid, sizeof L.grid);
     add(&L.smem, sizeof L.smem);
     add(&L.G, sizeof L.G);
+    add(&L.fma, sizeof L.fma);
     add(&L.VT, sizeof L.VT);
     add(&L.NW, sizeof L.NW);
     add(&L.col0, sizeof L.col0);

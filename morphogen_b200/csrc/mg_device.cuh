@@ -292,6 +292,7 @@ struct Segment {
   uint32_t g;           // keys per group (<= kernel G)
   uint32_t key_base;    // KeyDev index of group 0, key 0
   uint32_t col_base;    // partial column of group 0, key 0, lane 0
+  uint64_t fr_base;     // frontier index of group 0, key 0 (key j at fr_base + j * tiles)
 };
 
 struct ScanParams {
@@ -302,6 +303,8 @@ struct ScanParams {
   uint32_t nsegs;
   uint32_t cols;        // total share uint4s of the pass
   uint32_t slots;       // stack slots per key per thread allocated in smem
+  const uint4* fr_seed; // frontier holding every key's tile roots, or null: CTAs walk to them
+  const uint8_t* fr_t;
 };
 
 // ---- warp-independent scan ------------------------------------------------

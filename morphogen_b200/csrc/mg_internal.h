@@ -14,9 +14,10 @@ bool scan_g_supported(int G);
 // Raise (never lower) the kernel's dynamic shared memory limit on the current
 // device to at least smem.  The limit is process-wide per device and kernel,
 // so every caller goes through this one record (scan_prepare / warp_prepare).
-cudaError_t scan_prepare(int G, size_t smem);
-int scan_occupancy(int G, size_t smem);
-cudaError_t launch_scan(int G, const ScanParams& p, uint32_t grid, size_t smem, cudaStream_t st);
+bool scan_fma(uint32_t V);  // which of the kernel's two PRG forms rows of V uint4 take
+cudaError_t scan_prepare(int G, bool fma, size_t smem);
+int scan_occupancy(int G, bool fma, size_t smem);
+cudaError_t launch_scan(int G, bool fma, const ScanParams& p, uint32_t grid, size_t smem, cudaStream_t st);
 // out = XOR of the partial rows; out is cleared first unless out_zeroed.
 cudaError_t launch_reduce(const uint4* partial, uint32_t nparts, uint32_t cols, uint4* out,
                           cudaStream_t st, bool out_zeroed = false);

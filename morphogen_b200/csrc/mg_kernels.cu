@@ -2,8 +2,12 @@
 //
 // scan_kernel<G>: persistent CTAs walk a list of (tile, key group) work items.
 // For one item (an aligned subtree of 2^S rows and g <= G keys):
-//   1. threads 0..g-1 walk each key from its root to the tile root (d - S
-//      levels; the prefix walk of dpf.rs:183-203);
+//   1. each key's node at the tile root is read from a frontier, or, when a CTA
+//      has one item only, walked to from the key's root by threads 0..g-1 (d - S
+//      levels; the prefix walk of dpf.rs:183-203).  The walk's 16 serial levels
+//      and the barriers around them took 27k cycles per item, 10% of the time
+//      of a 512-page tile: 1300021 x 4 KB 940 us with it, 887 without (0.92 of
+//      the measured copy rate);
 //   2. the CTA expands U levels breadth-first in shared memory, giving every
 //      thread one node 2^M leaves above the rows (the GGM tree of
 //      dpf.rs:210-246 in breadth-first order);
@@ -33,7 +37,9 @@ namespace mg {
 
 // Up to 4 keys per CTA the kernel is held to 80 registers so that three
 // CTAs share an SM (page mode: more bytes in flight per SM).
-template <int G>
+// FMA: node expansions balanced over both integer pipes, or all-ALU (see
+// launch_scan).
+template <int G, bool FMA>
 __global__ void __launch_bounds__(kThreads, (G <= 4 ? 3 : 2)) scan_kernel(const __grid_constant__ ScanParams p) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   KeyDev* s_keys = reinterpret_cast<KeyDev*>(smem_raw);
@@ -64,27 +70,36 @@ __global__ void __launch_bounds__(kThreads, (G <= 4 ? 3 : 2)) scan_kernel(const 
       const uint32_t n = g * (uint32_t)(sizeof(KeyDev) / 16);
       for (uint32_t i = tid; i < n; i += kThreads) dst[i] = src[i];
     }
-    __syncthreads();
-
-    // 1. prefix walk to the tile root; the breadth-first ping-pong below
-    //    starts in slot (U & 1) so that it ends in slot 0.
+    // 1. the tile's root, from the frontier or by the prefix walk; the
+    //    breadth-first ping-pong below starts in slot (U & 1) so that it ends
+    //    in slot 0.
     const uint32_t start_slot = U & 1u;
-    if (tid < g) {
-      const KeyDev& K = s_keys[tid];
-      uint4 s = K.root_seed;
-      uint32_t t = K.root_t;
-      for (uint32_t lvl = 0; lvl < L0; ++lvl) {
-        uint4 Lc, Rc;
-        uint32_t tl, tr;
-        expand_cw<false>(s, t, K, lvl, Lc, tl, Rc, tr);
-        const uint32_t bit = (tile >> (L0 - 1 - lvl)) & 1u;
-        s = bit ? Rc : Lc;
-        t = bit ? tr : tl;
+    if (p.fr_seed) {
+      if (tid < g) {
+        const uint64_t at = sg.fr_base + ((uint64_t)group * g + tid) * sg.tiles + local / sg.groups;
+        s_seed[(tid * slots + start_slot) * kThreads] = p.fr_seed[at];
+        s_t[(tid * slots + start_slot) * kThreads] = p.fr_t[at];
       }
-      s_seed[(tid * slots + start_slot) * kThreads] = s;
-      s_t[(tid * slots + start_slot) * kThreads] = (uint8_t)t;
+      __syncthreads();
+    } else {
+      __syncthreads();
+      if (tid < g) {
+        const KeyDev& K = s_keys[tid];
+        uint4 s = K.root_seed;
+        uint32_t t = K.root_t;
+        for (uint32_t lvl = 0; lvl < L0; ++lvl) {
+          uint4 Lc, Rc;
+          uint32_t tl, tr;
+          expand_cw<false>(s, t, K, lvl, Lc, tl, Rc, tr);
+          const uint32_t bit = (tile >> (L0 - 1 - lvl)) & 1u;
+          s = bit ? Rc : Lc;
+          t = bit ? tr : tl;
+        }
+        s_seed[(tid * slots + start_slot) * kThreads] = s;
+        s_t[(tid * slots + start_slot) * kThreads] = (uint8_t)t;
+      }
+      __syncthreads();
     }
-    __syncthreads();
 
     // 2. breadth-first expansion of U levels below the tile root.
     uint32_t cur = start_slot;
@@ -97,7 +112,7 @@ __global__ void __launch_bounds__(kThreads, (G <= 4 ? 3 : 2)) scan_kernel(const 
         const size_t dst = (k * slots + nxt) * kThreads + 2 * i;
         uint4 Lc, Rc;
         uint32_t tl, tr;
-        expand_cw(s_seed[src], s_t[src], s_keys[k], L0 + j, Lc, tl, Rc, tr);
+        expand_cw<FMA>(s_seed[src], s_t[src], s_keys[k], L0 + j, Lc, tl, Rc, tr);
         s_seed[dst] = Lc;
         s_seed[dst + 1] = Rc;
         s_t[dst] = (uint8_t)tl;
@@ -146,7 +161,7 @@ __global__ void __launch_bounds__(kThreads, (G <= 4 ? 3 : 2)) scan_kernel(const 
           for (;; ++lvl) {
             uint4 Lc, Rc;
             uint32_t tl, tr;
-            expand_cw(s, t, K, abs0 + lvl, Lc, tl, Rc, tr);
+            expand_cw<FMA>(s, t, K, abs0 + lvl, Lc, tl, Rc, tr);
             if (lvl == M - 1) {
               mk[0] = leaf_mask(Lc, tl, K);
               mk[1] = leaf_mask(Rc, tr, K);
@@ -1132,54 +1147,45 @@ size_t scan_smem_bytes(int G, uint32_t slots) {
   return (size_t)G * (sizeof(KeyDev) + 2 * kThreads * 16 + (size_t)slots * kThreads * 17);
 }
 
-template <int G>
-static cudaError_t launch_scan_t(const ScanParams& p, uint32_t grid, size_t smem, cudaStream_t st) {
-  scan_kernel<G><<<grid, kThreads, smem, st>>>(p);
-  return cudaGetLastError();
-}
-
-template <int G>
-static cudaError_t prepare_t(size_t smem) {
-  return raise_smem_limit(reinterpret_cast<const void*>(scan_kernel<G>), smem);
-}
-
-template <int G>
-static int occupancy_t(size_t smem) {
-  int n = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, scan_kernel<G>, kThreads, smem) != cudaSuccess)
-    return 0;
-  return n;
-}
-
-#define MG_G_DISPATCH(G_, EXPR1, EXPR2, EXPR3, EXPR4, EXPR8) \
-  switch (G_) {                                              \
-    case 1: return EXPR1;                                    \
-    case 2: return EXPR2;                                    \
-    case 3: return EXPR3;                                    \
-    case 4: return EXPR4;                                    \
-    case 8: return EXPR8;                                    \
-    default: break;                                          \
+using ScanKernel = void (*)(const ScanParams);
+template <bool FMA>
+static ScanKernel scan_kernel_of(int G) {
+  switch (G) {
+    case 1: return scan_kernel<1, FMA>;
+    case 2: return scan_kernel<2, FMA>;
+    case 3: return scan_kernel<3, FMA>;
+    case 4: return scan_kernel<4, FMA>;
+    case 8: return scan_kernel<8, FMA>;
+    default: return nullptr;
   }
+}
+static ScanKernel scan_kernel_of(int G, bool fma) { return fma ? scan_kernel_of<true>(G) : scan_kernel_of<false>(G); }
 
 bool scan_g_supported(int G) { return G == 1 || G == 2 || G == 3 || G == 4 || G == 8; }
 
-cudaError_t scan_prepare(int G, size_t smem) {
-  MG_G_DISPATCH(G, prepare_t<1>(smem), prepare_t<2>(smem), prepare_t<3>(smem), prepare_t<4>(smem),
-                prepare_t<8>(smem));
-  return cudaErrorInvalidValue;
+cudaError_t scan_prepare(int G, bool fma, size_t smem) {
+  const ScanKernel k = scan_kernel_of(G, fma);
+  return k ? raise_smem_limit(reinterpret_cast<const void*>(k), smem) : cudaErrorInvalidValue;
 }
 
-int scan_occupancy(int G, size_t smem) {
-  MG_G_DISPATCH(G, occupancy_t<1>(smem), occupancy_t<2>(smem), occupancy_t<3>(smem),
-                occupancy_t<4>(smem), occupancy_t<8>(smem));
-  return 0;
+int scan_occupancy(int G, bool fma, size_t smem) {
+  const ScanKernel k = scan_kernel_of(G, fma);
+  int n = 0;
+  if (!k || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, kThreads, smem) != cudaSuccess) return 0;
+  return n;
 }
 
-cudaError_t launch_scan(int G, const ScanParams& p, uint32_t grid, size_t smem, cudaStream_t st) {
-  MG_G_DISPATCH(G, launch_scan_t<1>(p, grid, smem, st), launch_scan_t<2>(p, grid, smem, st),
-                launch_scan_t<3>(p, grid, smem, st), launch_scan_t<4>(p, grid, smem, st),
-                launch_scan_t<8>(p, grid, smem, st));
-  return cudaErrorInvalidValue;
+// Rows under 2 KB leave the pass bound by its node expansions as much as by
+// memory, and the balanced PRG is faster (3 keys, 10^6 x 528 B: 239 us against
+// 252); wider ones are bound by HBM and its power, where the all-ALU form with
+// fewer instructions wins (1300021 x 4 KB: 887 us against 925).
+bool scan_fma(uint32_t V) { return V < 128; }
+
+cudaError_t launch_scan(int G, bool fma, const ScanParams& p, uint32_t grid, size_t smem, cudaStream_t st) {
+  const ScanKernel k = scan_kernel_of(G, fma);
+  if (!k) return cudaErrorInvalidValue;
+  k<<<grid, kThreads, smem, st>>>(p);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_reduce(const uint4* partial, uint32_t nparts, uint32_t cols, uint4* out,

@@ -145,6 +145,7 @@ extern "C" int mg_scan_noalloc(int device, const void* table_dev, uint64_t rows,
 
   // Shape: one key per CTA, the deepest tile (<= 14 levels) giving >= 4 waves.
   const uint32_t V = row_bytes / 16;
+  const bool fma = mg::scan_fma(V);
   mg::ScanParams p;
   std::memset(&p, 0, sizeof p);
   uint32_t grid = 0;
@@ -159,9 +160,9 @@ extern "C" int mg_scan_noalloc(int device, const void* table_dev, uint64_t rows,
     const uint64_t items = tiles * nkeys;
     int occ = 0;
     if (smem <= slot->smem_optin) {
-      if (mg::scan_prepare(1, smem) != cudaSuccess)
+      if (mg::scan_prepare(1, fma, smem) != cudaSuccess)
         return noalloc_fail(MG_ECUDA, "mg_scan_noalloc: cannot set the kernel's shared memory");
-      occ = mg::scan_occupancy(1, smem);
+      occ = mg::scan_occupancy(1, fma, smem);
     }
     const uint64_t slots_total = (uint64_t)(occ > 0 ? occ : 1) * slot->sms;
     if ((occ > 0 && items >= 4 * slots_total) || S_target <= 8) {
@@ -210,7 +211,7 @@ extern "C" int mg_scan_noalloc(int device, const void* table_dev, uint64_t rows,
     stage_keys_kernel<<<1, 256, 0, st>>>(ks, d_keys + i0);
     if (cudaGetLastError() != cudaSuccess) return noalloc_fail(MG_ECUDA, "mg_scan_noalloc: key upload failed");
   }
-  if (mg::launch_scan(1, p, grid, smem, st) != cudaSuccess)
+  if (mg::launch_scan(1, fma, p, grid, smem, st) != cudaSuccess)
     return noalloc_fail(MG_ECUDA, "mg_scan_noalloc: scan launch failed");
   if (mg::launch_reduce(p.partial, grid, p.cols, static_cast<uint4*>(out_shares_dev), st) != cudaSuccess)
     return noalloc_fail(MG_ECUDA, "mg_scan_noalloc: reduction launch failed");

@@ -106,3 +106,24 @@ def test_frontier_levels_per_cta(scanner, oracle_mod, d, M, first, nrows):
     assert ws.read() == oracle_mod.scan_fused(keys, host, 16, row_base=first)
     ws.close()
     db.close()
+
+
+@pytest.mark.parametrize("row_bytes,keys_per_cta", [(528, 1), (528, 3), (1024, 2), (2048, 4), (1040, 8)])
+def test_cta_kernel_with_several_tiles_per_cta(scanner, oracle_mod, row_bytes, keys_per_cta):
+    # More tiles than CTAs: the tiles' roots come from a frontier.
+    d, first, nrows, nkeys = 24, 1_000_001, 120_007, 9
+    db = G.GpuPageMatrix.from_seed(scanner, nrows, row_bytes, seed=7, first_row=first)
+    host = oracle_mod.fill_splitmix(first * row_bytes, nrows * row_bytes, 7).reshape(nrows, row_bytes)
+    keys = [oracle_keypair(oracle_mod, d, first + (7919 * j) % nrows, seed=94, i=j)[0] for j in range(nkeys)]
+    ws = scanner.workspace()
+    ws.set_kernel("cta")
+    ws.set_shape(8, keys_per_cta)
+    ws.set_keys([db] * nkeys, keys)
+    plan = ws.plan()
+    assert plan["kernel"] == N.KERNEL_CTA and plan["items"] > plan["grid"] and plan["frontier_nodes"] > 0
+    want = oracle_mod.scan_fused(keys, host, row_bytes, row_base=first)
+    for graph in (False, True):
+        ws.launch(graph=graph)
+        assert ws.read() == want
+    ws.close()
+    db.close()
