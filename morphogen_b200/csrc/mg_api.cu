@@ -226,8 +226,8 @@ struct mg_batch {
     uint32_t job0, njobs;  // range in d_jobs
   };
   std::vector<DeltaLaunch> deltas;
-  uint2* d_jobs = nullptr;
-  uint2* h_jobs = nullptr;
+  mg::DeltaJob* d_jobs = nullptr;
+  mg::DeltaJob* h_jobs = nullptr;
   size_t cap_jobs = 0;
   uint32_t total_cols = 0;
   std::vector<uint32_t> key_col;    // first share column of input key i
@@ -1127,13 +1127,39 @@ static int enqueue_pass(mg_batch* b, cudaStream_t st, cudaEvent_t mark, bool out
       MG_CUDA(mg::launch_reduce(b->d_partial, L.nparts, L.cols, b->d_out + L.col0, st, out_zeroed));
   }
   for (const mg_batch::DeltaLaunch& dl : b->deltas)
-    MG_CUDA(mg::launch_delta(b->d_keys, b->d_jobs + dl.job0, dl.njobs, dl.table->d_delta_idx, dl.table->d_delta_diff,
+    MG_CUDA(mg::launch_delta(b->d_keys, b->d_jobs + dl.job0, dl.njobs, b->d_fr_seed, b->d_fr_t, dl.table->d_delta_idx, dl.table->d_delta_diff,
                              dl.table->d_delta_count, dl.table->delta_cap, dl.table->row_bytes / 16, dl.table->first,
                              b->d_out, st));
   return MG_OK;
 }
 
 namespace {
+
+// The delta job of the key in slot `slot`: its segment's frontier, if the pass
+// computes one.
+mg::DeltaJob delta_job(const std::vector<mg_batch::Launch>& launches, const mg_table* t, uint32_t slot, uint32_t col) {
+  mg::DeltaJob job;
+  std::memset(&job, 0, sizeof job);
+  job.key = slot;
+  job.col = col;
+  job.below = ~0u;
+  auto found = [&](uint32_t key_base, uint32_t keys, uint32_t below, uint64_t fr_base, uint64_t nodes) {
+    if (slot < key_base || slot >= key_base + keys || nodes == 0) return false;
+    job.below = below;
+    job.fr_base = fr_base + (slot - key_base) * nodes;
+    job.fr_first = level_first(t, below);
+    return true;
+  };
+  for (const mg_batch::Launch& L : launches) {
+    if (L.steps.empty()) continue;
+    for (uint32_t s = 0; s < (L.kind == MG_KERNEL_CTA ? L.p.nsegs : L.w.nsegs); ++s)
+      if (L.kind == MG_KERNEL_CTA
+              ? found(L.p.seg[s].key_base, L.p.seg[s].groups * L.p.seg[s].g, L.p.seg[s].S, L.p.seg[s].fr_base, L.p.seg[s].tiles)
+              : found(L.w.seg[s].key_base, L.w.seg[s].groups * L.w.seg[s].g, L.w.seg[s].M, L.w.seg[s].fr_base, L.w.seg[s].nF))
+        return job;
+  }
+  return job;
+}
 
 // Plan the pass for b->in_keys / b->in_tables with the effective shape
 // (b->eff_kind, b->eff_S, b->eff_G), allocate, stage the keys and copy them
@@ -1228,7 +1254,7 @@ int plan_pass(mg_batch* b) {
 
   // Delta folding: one launch per table that holds a delta buffer.
   std::vector<mg_batch::DeltaLaunch> deltas;
-  std::vector<uint2> jobs;
+  std::vector<mg::DeltaJob> jobs;
   for (uint32_t i = 0; i < nkeys; ++i) {
     const mg_table* t = b->in_tables[i];
     if (!t->delta_cap) continue;
@@ -1241,7 +1267,7 @@ int plan_pass(mg_batch* b) {
   for (mg_batch::DeltaLaunch& dl : deltas) {
     dl.job0 = (uint32_t)jobs.size();
     for (uint32_t i = 0; i < nkeys; ++i)
-      if (b->in_tables[i] == dl.table) jobs.push_back(make_uint2(key_slot[i], key_col[i]));
+      if (b->in_tables[i] == dl.table) jobs.push_back(delta_job(launches, dl.table, key_slot[i], key_col[i]));
     dl.njobs = (uint32_t)jobs.size() - dl.job0;
   }
   if (jobs.size() > b->cap_jobs) {
@@ -1250,16 +1276,16 @@ int plan_pass(mg_batch* b) {
     b->d_jobs = nullptr;
     b->h_jobs = nullptr;
     b->cap_jobs = 0;
-    if (cudaMalloc(&b->d_jobs, jobs.size() * sizeof(uint2)) != cudaSuccess ||
-        cudaMallocHost(&b->h_jobs, jobs.size() * sizeof(uint2)) != cudaSuccess) {
+    if (cudaMalloc(&b->d_jobs, jobs.size() * sizeof(mg::DeltaJob)) != cudaSuccess ||
+        cudaMallocHost(&b->h_jobs, jobs.size() * sizeof(mg::DeltaJob)) != cudaSuccess) {
       cudaGetLastError();
       return fail(MG_ENOMEM, "cannot allocate delta job lists");
     }
     b->cap_jobs = jobs.size();
   }
   if (!jobs.empty()) {
-    std::memcpy(b->h_jobs, jobs.data(), jobs.size() * sizeof(uint2));
-    MG_CUDA(cudaMemcpyAsync(b->d_jobs, b->h_jobs, jobs.size() * sizeof(uint2), cudaMemcpyHostToDevice, b->stream));
+    std::memcpy(b->h_jobs, jobs.data(), jobs.size() * sizeof(mg::DeltaJob));
+    MG_CUDA(cudaMemcpyAsync(b->d_jobs, b->h_jobs, jobs.size() * sizeof(mg::DeltaJob), cudaMemcpyHostToDevice, b->stream));
   }
   b->deltas = std::move(deltas);
 
@@ -1606,6 +1632,7 @@ std::vector<uint8_t> pass_signature(const mg_batch* b) {
     add(&dl.table->delta_cap, sizeof dl.table->delta_cap);
   }
   add(&b->d_out, sizeof b->d_out);
+  add(&b->d_fr_seed, sizeof b->d_fr_seed);
   return sig;
 }
 

@@ -367,6 +367,17 @@ struct WarpScanParams {
   uint32_t queues;      // item queues per CTA: 1, or 4 (one per warp scheduler)
 };
 
+// A key whose table has a pending delta: its key slot, its first share column
+// and, when the pass holds a frontier for it, where that is.
+struct DeltaJob {
+  uint32_t key;
+  uint32_t col;
+  uint32_t below;      // levels from the frontier's nodes to the leaves; ~0: no frontier
+  uint32_t pad;
+  uint64_t fr_base;    // frontier index of the key's node 0
+  uint64_t fr_first;   // level index of node 0
+};
+
 // Most levels one frontier-chain step expands: breadth first up to
 // kFrontierWide (one node per thread of its CTA), the rest depth first.
 constexpr uint32_t kFrontierWide = 8;

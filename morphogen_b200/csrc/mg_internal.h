@@ -44,8 +44,9 @@ bool warp_reduces_in_kernel(int G, uint32_t V);
 cudaError_t launch_scan_warp(int G, uint32_t V, const WarpScanParams& p, uint32_t grid, uint32_t nw, size_t smem,
                              cudaStream_t st);
 cudaError_t launch_frontier(const FrontierStep& f, uint32_t nkeys, cudaStream_t st);
-// Folds a table's pending delta into the shares: jobs[j] = (key slot, first share column).
-cudaError_t launch_delta(const KeyDev* keys, const uint2* jobs, uint32_t njobs, const uint64_t* idx,
+// Folds a table's pending delta into the shares of its keys (jobs).
+cudaError_t launch_delta(const KeyDev* keys, const DeltaJob* jobs, uint32_t njobs, const uint4* fr_seed,
+                         const uint8_t* fr_t, const uint64_t* idx,
                          const void* diffs, const uint32_t* count, uint32_t capacity, uint32_t V, uint64_t first,
                          uint4* out, cudaStream_t st);
 

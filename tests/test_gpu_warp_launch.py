@@ -3,6 +3,7 @@ at a time (one pair only at depth 1), CTAs from one warp to the full width as
 the items go from fewer than the SMs to several rounds per warp, and the block
 scan over row sizes, depths and key groups.  Shares are
 exact: the oracle's bytes."""
+import numpy as np
 import pytest
 
 from conftest import oracle_keypair
@@ -121,6 +122,34 @@ def test_cta_kernel_with_several_tiles_per_cta(scanner, oracle_mod, row_bytes, k
     ws.set_keys([db] * nkeys, keys)
     plan = ws.plan()
     assert plan["kernel"] == N.KERNEL_CTA and plan["items"] > plan["grid"] and plan["frontier_nodes"] > 0
+    want = oracle_mod.scan_fused(keys, host, row_bytes, row_base=first)
+    for graph in (False, True):
+        ws.launch(graph=graph)
+        assert ws.read() == want
+    ws.close()
+    db.close()
+
+
+@pytest.mark.parametrize("row_bytes,nrows,kind", [(32, 70_001, "auto"), (48, 20_011, "auto"), (256, 9_001, "auto"),
+                                                  (4096, 300, "auto"), (528, 120_007, "cta"), (64, 33, "auto")])
+def test_delta_entries_start_from_the_pass_frontier(scanner, oracle_mod, row_bytes, nrows, kind):
+    # Pending entries (first and last row, duplicates) are evaluated from their
+    # rows' ancestors in the frontier, or from the root when the pass has none.
+    d, first = 23, 4_000_003
+    db = G.GpuPageMatrix.from_seed(scanner, nrows, row_bytes, seed=8, first_row=first)
+    host = oracle_mod.fill_splitmix(first * row_bytes, nrows * row_bytes, 8).reshape(nrows, row_bytes).copy()
+    keys = [oracle_keypair(oracle_mod, d, first + (7919 * j) % nrows, seed=95, i=j)[0] for j in range(4)]
+    rng = np.random.default_rng(row_bytes)
+    idx = np.concatenate([[0, nrows - 1, nrows // 2, nrows // 2], rng.integers(0, nrows, 700)]).astype(np.uint64)
+    diffs = rng.integers(0, 256, idx.size * row_bytes, dtype=np.uint8).reshape(-1, row_bytes)
+    np.bitwise_xor.at(host, idx.astype(np.int64), diffs)
+    db.delta_reserve(1000)
+    db.delta_push(idx, diffs)
+    ws = scanner.workspace()
+    ws.set_kernel(kind)
+    if kind == "cta":
+        ws.set_shape(8, 3)
+    ws.set_keys([db] * 4, keys)
     want = oracle_mod.scan_fused(keys, host, row_bytes, row_base=first)
     for graph in (False, True):
         ws.launch(graph=graph)
