@@ -35,12 +35,22 @@
 
 namespace mg {
 
+// Every kernel of a pass begins with this: it lets the pass's next kernel be
+// launched while this one runs (its CTAs take their places as these leave) and
+// then waits until the kernel before it has completed and its writes are
+// visible.  Nothing in global memory is touched earlier.  See launch_chained.
+__device__ __forceinline__ void chain_begin() {
+  cudaTriggerProgrammaticLaunchCompletion();
+  cudaGridDependencySynchronize();
+}
+
 // Up to 4 keys per CTA the kernel is held to 80 registers so that three
 // CTAs share an SM (page mode: more bytes in flight per SM).
 // FMA: node expansions balanced over both integer pipes, or all-ALU (see
 // launch_scan).
 template <int G, bool FMA>
 __global__ void __launch_bounds__(kThreads, (G <= 4 ? 3 : 2)) scan_kernel(const __grid_constant__ ScanParams p) {
+  chain_begin();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   KeyDev* s_keys = reinterpret_cast<KeyDev*>(smem_raw);
   uint4* s_mask = reinterpret_cast<uint4*>(smem_raw + G * sizeof(KeyDev));  // [G][2*T]
@@ -275,6 +285,7 @@ __global__ void __launch_bounds__(kThreads, (G <= 4 ? 3 : 2)) scan_kernel(const 
 // last c - 8 levels are walked depth first, one of the 256 nodes per thread,
 // with no barrier at all.
 __global__ void __launch_bounds__(kThreads) frontier_kernel(const __grid_constant__ FrontierStep f) {
+  chain_begin();
   constexpr uint32_t kWide = 1u << kFrontierWide;  // nodes of the widest breadth-first level
   static_assert(kWide == kThreads, "one node per thread for the depth-first levels");
   __shared__ uint4 sa[kWide], sb[kWide];
@@ -564,10 +575,11 @@ __global__ void __launch_bounds__(warp_cta_warps(1) * 32, 1) scan_pair_kernel(co
   const LaneStack st = {stk4 + (size_t)warp * p.slots * 32 + lane,
                         reinterpret_cast<int8_t*>(stk4 + (size_t)nw * p.slots * 32) + (size_t)warp * p.slots * 32 + lane};
   uint4* const my_partial = p.partial + ((uint64_t)blockIdx.x * nw + warp) * p.cols;
-  for (uint32_t c = lane; c < p.cols; c += 32) my_partial[c] = make_uint4(0u, 0u, 0u, 0u);
   const ItemQueue queue(p, s_next, warp, nw);
   if (threadIdx.x < 4) s_next[threadIdx.x] = 0;
   __syncthreads();
+  chain_begin();
+  for (uint32_t c = lane; c < p.cols; c += 32) my_partial[c] = make_uint4(0u, 0u, 0u, 0u);
 
   uint4 acc[AV];
 #pragma unroll
@@ -682,6 +694,7 @@ __global__ void __launch_bounds__(warp_cta_warps(1) * 32, 1) scan_pair_kernel(co
 template <int G, int VT>
 __global__ void __launch_bounds__(warp_cta_warps(G) * 32, 1)
     scan_block_kernel(const __grid_constant__ WarpScanParams p) {
+  chain_begin();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ uint32_t s_next[4];  // next item of each scheduler's queue
   constexpr uint32_t kRows = 32u * kBlockLeaves;
@@ -920,6 +933,7 @@ bool warp_reduces_in_kernel(int G, uint32_t V) { return G > 1 || V > 2; }
 __global__ void __launch_bounds__(kThreads) reduce_kernel(const uint4* __restrict__ partial,
                                                           uint32_t nparts, uint32_t cols,
                                                           uint32_t per_block, uint4* __restrict__ out) {
+  chain_begin();
   __shared__ uint4 red[kThreads];
   const uint32_t cpb = cols < 32u ? cols : 32u;
   const uint32_t slices = kThreads / cpb;
@@ -972,6 +986,7 @@ __global__ void __launch_bounds__(kThreads) delta_kernel(const KeyDev* __restric
                                                          const uint64_t* __restrict__ idx, const uint4* __restrict__ diffs,
                                                          const uint32_t* __restrict__ count, uint32_t V, uint64_t first,
                                                          uint4* __restrict__ out) {
+  chain_begin();
   __shared__ uint4 s_acc[MG_MAX_ROW_BYTES / 16];
   const uint32_t n = *count;
   const uint64_t e0 = (uint64_t)blockIdx.x * kThreads;
@@ -1046,6 +1061,7 @@ __global__ void fill_splitmix_kernel(uint2* __restrict__ dst, uint64_t words, ui
 // sooner than a copy-engine transfer of a few KB.
 __global__ void copy_u4_kernel(const uint4* __restrict__ src, uint4* __restrict__ dst, uint32_t n,
                                uint4* __restrict__ zero, uint32_t nz) {
+  chain_begin();
   const uint32_t m = n > nz ? n : nz;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) {
     if (i < n) dst[i] = src[i];
@@ -1117,6 +1133,27 @@ __global__ void __launch_bounds__(256) prg_peak_kernel(uint32_t* __restrict__ ou
 }
 
 // ---- host-side launchers --------------------------------------------------
+
+// Launch a kernel that begins with chain_begin(): when the work before it on
+// the stream is such a kernel too, it need not have completed for this one's
+// launch to be processed (programmatic stream serialization; a captured graph
+// gets programmatic edges).  One call of five kernels, 4099 x 32 B: 49.5 us
+// without, 46.0 with; 1300021 x 4 KB pages, launched directly: 998 and 981.
+template <class... P, class... A>
+static cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, uint32_t threads, size_t smem, cudaStream_t st,
+                                  A&&... args) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+}
 
 // The dynamic shared memory limit of a kernel (cudaFuncAttributeMax-
 // DynamicSharedMemorySize) belongs to the kernel function on its device, for
@@ -1197,8 +1234,7 @@ bool scan_fma(uint32_t V) { return V < 128; }
 cudaError_t launch_scan(int G, bool fma, const ScanParams& p, uint32_t grid, size_t smem, cudaStream_t st) {
   const ScanKernel k = scan_kernel_of(G, fma);
   if (!k) return cudaErrorInvalidValue;
-  k<<<grid, kThreads, smem, st>>>(p);
-  return cudaGetLastError();
+  return launch_chained(k, dim3(grid), kThreads, smem, st, p);
 }
 
 cudaError_t launch_reduce(const uint4* partial, uint32_t nparts, uint32_t cols, uint4* out,
@@ -1210,17 +1246,15 @@ cudaError_t launch_reduce(const uint4* partial, uint32_t nparts, uint32_t cols, 
   const uint32_t slices = kThreads / cpb;
   const uint32_t per_block = slices * 4;  // at most 4 partial rows per thread
   const dim3 grid((cols + cpb - 1) / cpb, nparts ? (nparts + per_block - 1) / per_block : 1);
-  reduce_kernel<<<grid, kThreads, 0, st>>>(partial, nparts, cols, per_block, out);
-  return cudaGetLastError();
+  return launch_chained(reduce_kernel, grid, kThreads, 0, st, partial, nparts, cols, per_block, out);
 }
 
 cudaError_t launch_copy_u4(const void* src, void* dst, uint32_t n, cudaStream_t st, void* zero, uint32_t nz) {
   const uint32_t m = n > nz ? n : nz;
   if (m == 0) return cudaSuccess;
   const uint32_t blocks = (m + kThreads - 1) / kThreads < 32u ? (m + kThreads - 1) / kThreads : 32u;
-  copy_u4_kernel<<<blocks, kThreads, 0, st>>>(static_cast<const uint4*>(src), static_cast<uint4*>(dst), n,
-                                              static_cast<uint4*>(zero), nz);
-  return cudaGetLastError();
+  return launch_chained(copy_u4_kernel, dim3(blocks), kThreads, 0, st, static_cast<const uint4*>(src),
+                        static_cast<uint4*>(dst), n, static_cast<uint4*>(zero), nz);
 }
 
 cudaError_t launch_fill_splitmix(void* dst, uint64_t words, uint64_t seed, uint64_t word0, int sms, cudaStream_t st) {
@@ -1307,8 +1341,7 @@ cudaError_t launch_scan_warp(int G, uint32_t V, const WarpScanParams& p, uint32_
                              cudaStream_t st) {
   const WarpKernel k = warp_kernel(G, V);
   if (!k) return cudaErrorInvalidValue;
-  k<<<grid, nw * 32, smem, st>>>(p);
-  return cudaGetLastError();
+  return launch_chained(k, dim3(grid), nw * 32, smem, st, p);
 }
 
 cudaError_t launch_delta(const KeyDev* keys, const DeltaJob* jobs, uint32_t njobs, const uint4* fr_seed,
@@ -1317,17 +1350,15 @@ cudaError_t launch_delta(const KeyDev* keys, const DeltaJob* jobs, uint32_t njob
                          uint4* out, cudaStream_t st) {
   if (njobs == 0 || capacity == 0) return cudaSuccess;
   dim3 grid((capacity + kThreads - 1) / kThreads, njobs);
-  delta_kernel<<<grid, kThreads, 0, st>>>(keys, jobs, fr_seed, fr_t, idx, reinterpret_cast<const uint4*>(diffs), count, V, first,
-                                          out);
-  return cudaGetLastError();
+  return launch_chained(delta_kernel, grid, kThreads, 0, st, keys, jobs, fr_seed, fr_t, idx,
+                        static_cast<const uint4*>(diffs), count, V, first, out);
 }
 
 cudaError_t launch_frontier(const FrontierStep& f, uint32_t nkeys, cudaStream_t st) {
   if (f.n_in == 0 || nkeys == 0) return cudaSuccess;
   if (f.c > kFrontierLevels || f.L_in + f.c > (uint32_t)kMaxLevels) return cudaErrorInvalidValue;
   dim3 grid((unsigned)f.n_in, nkeys);
-  frontier_kernel<<<grid, kThreads, 0, st>>>(f);
-  return cudaGetLastError();
+  return launch_chained(frontier_kernel, grid, kThreads, 0, st, f);
 }
 
 }  // namespace mg
