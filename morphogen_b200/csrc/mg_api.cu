@@ -864,7 +864,10 @@ size_t wire_frontier(mg_batch* b, mg_batch::Launch& L, size_t st, uint32_t F, ui
 }
 
 // Plan one CTA-kernel launch over segs (at most kMaxSegs): tile depth S, the
-// deepest in [8, 14] that still gives >= 4 waves of items (or the pinned one).
+// deepest in [8, 14] that still gives >= 4 waves of items (or the pinned one);
+// for a small table, which at S = 8 would leave SMs idle, the shallowest that
+// still is one wave (3 keys, 10225 x 4 KB: 33 us at S = 5, 42 at 4, 61 at 8;
+// 30000 x 4 KB: 54 at 7, 67 at 6, 61 at 8).
 int plan_cta(mg_batch* b, const std::vector<SegPlan>& segs, int G, uint32_t col0, size_t& key_cursor,
              std::vector<uint32_t>& key_col, std::vector<uint32_t>& key_bytes, std::vector<uint32_t>& key_slot,
              uint64_t& fr_cursor, size_t& tmp_need, mg_batch::Launch& out) {
@@ -925,8 +928,9 @@ int plan_cta(mg_batch* b, const std::vector<SegPlan>& segs, int G, uint32_t col0
       occ = mg::scan_occupancy(G, L.fma, L.smem);
     }
     const uint64_t slots_total = (uint64_t)std::max(occ, 1) * ctx->sms;
-    const bool enough = occ > 0 && items >= 4 * slots_total;
-    if (b->eff_S || enough || S_target <= 8) {
+    const bool enough = S_target >= 8 && occ > 0 && items >= 4 * slots_total;
+    const bool full = S_target <= 8 && (2 * items > slots_total || S_target <= 3);
+    if (b->eff_S || enough || full) {
       if (occ <= 0) return fail(MG_EINVAL, "launch shape S=%u G=%d does not fit the device", S_target, G);
       L.grid = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(items, slots_total));
       L.nparts = L.grid;
