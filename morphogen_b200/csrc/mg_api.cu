@@ -206,6 +206,8 @@ struct mg_batch {
   int device = 0;
   cudaStream_t stream = nullptr;
   cudaEvent_t ev_k0 = nullptr, ev_km = nullptr, ev_k1 = nullptr, ev_done = nullptr, ev_h0 = nullptr, ev_h1 = nullptr;
+  void* d_arena = nullptr;  // one allocation each for all device and pinned buffers below
+  void* h_arena = nullptr;
   KeyDev* d_keys = nullptr;
   KeyDev* h_keys = nullptr;
   size_t cap_keys = 0;
@@ -293,63 +295,65 @@ int prepare_warp(mg_context* ctx, int G, uint32_t VT, size_t smem) {
   return MG_OK;
 }
 
-template <class T>
-int grow_dev(T*& p, size_t& cap, size_t need, const char* what) {
-  if (need <= cap) return MG_OK;
-  if (p) cudaFree(p);
-  p = nullptr;
-  cap = 0;
-  if (cudaMalloc(&p, need * sizeof(T)) != cudaSuccess) {
-    cudaGetLastError();
-    return fail(MG_ENOMEM, "cannot allocate %zu bytes of %s", need * sizeof(T), what);
-  }
-  cap = need;
-  return MG_OK;
-}
-
+// Room for a pass: every device buffer of the workspace is a part of one
+// allocation, both pinned ones parts of another, because the first pass of a
+// workspace pays for each call of cudaMalloc (about 0.1 ms; five to nine of
+// them took 0.4 of the 0.7 ms of a first call over 1000003 x 48 B).
 int grow(mg_batch* b, size_t nkeys, size_t partial_u4, size_t out_u4, size_t fr_nodes, size_t tmp_nodes) {
-  if (nkeys > b->cap_keys) {
-    if (b->d_keys) cudaFree(b->d_keys);
-    if (b->h_keys) cudaFreeHost(b->h_keys);
-    b->d_keys = nullptr;
-    b->h_keys = nullptr;
-    b->cap_keys = 0;
-    // Keys, then their warp-kernel constants (KeyAux) right after the pass's keys.
-    const size_t bytes = nkeys * (sizeof(KeyDev) + sizeof(mg::KeyAux));
-    if (cudaMalloc(&b->d_keys, bytes) != cudaSuccess || cudaMallocHost(&b->h_keys, bytes) != cudaSuccess) {
-      cudaGetLastError();
-      return fail(MG_ENOMEM, "cannot allocate key buffers for %zu keys", nkeys);
-    }
-    b->cap_keys = nkeys;
+  if (nkeys <= b->cap_keys && partial_u4 <= b->cap_partial && out_u4 <= b->cap_out && fr_nodes <= b->cap_fr &&
+      tmp_nodes <= b->cap_tmp)
+    return MG_OK;
+  nkeys = std::max(nkeys, b->cap_keys);
+  partial_u4 = std::max(partial_u4, b->cap_partial);
+  out_u4 = std::max(out_u4, b->cap_out);
+  fr_nodes = std::max(fr_nodes, b->cap_fr);
+  tmp_nodes = std::max(tmp_nodes, b->cap_tmp);
+  if (b->d_arena) cudaFree(b->d_arena);
+  if (b->h_arena) cudaFreeHost(b->h_arena);
+  b->d_arena = nullptr;
+  b->h_arena = nullptr;
+  b->cap_keys = b->cap_partial = b->cap_out = b->cap_fr = b->cap_tmp = 0;
+  size_t bytes = 0;
+  auto part = [&](size_t n) {
+    const size_t at = bytes;
+    bytes += (n + 255) / 256 * 256;
+    return at;
+  };
+  // Keys, then their warp-kernel constants (KeyAux) right after the pass's keys.
+  const size_t key_bytes = nkeys * (sizeof(KeyDev) + sizeof(mg::KeyAux));
+  const size_t keys_at = part(key_bytes), out_at = part(out_u4 * 16);
+  const size_t host_bytes = bytes;
+  const size_t partial_at = part(partial_u4 * 16), fr_at = part(fr_nodes * 16), fr_t_at = part(fr_nodes);
+  size_t tmp_at[2], tmp_t_at[2];
+  for (int i = 0; i < 2; ++i) {
+    tmp_at[i] = part(tmp_nodes * 16);
+    tmp_t_at[i] = part(tmp_nodes);
   }
-  if (int rc = grow_dev(b->d_partial, b->cap_partial, partial_u4, "partial rows")) return rc;
-  if (out_u4 > b->cap_out) {
-    if (b->d_out) cudaFree(b->d_out);
-    if (b->h_out) cudaFreeHost(b->h_out);
-    b->d_out = nullptr;
-    b->h_out = nullptr;
-    b->cap_out = 0;
-    if (cudaMalloc(&b->d_out, out_u4 * 16) != cudaSuccess ||
-        cudaMallocHost(&b->h_out, out_u4 * 16) != cudaSuccess) {
-      cudaGetLastError();
-      return fail(MG_ENOMEM, "cannot allocate share buffers (%zu bytes)", out_u4 * 16);
-    }
-    b->cap_out = out_u4;
+  if (cudaMalloc(&b->d_arena, bytes) != cudaSuccess || cudaMallocHost(&b->h_arena, host_bytes) != cudaSuccess) {
+    cudaGetLastError();
+    if (b->d_arena) cudaFree(b->d_arena);
+    b->d_arena = nullptr;
+    b->h_arena = nullptr;
+    return fail(MG_ENOMEM, "cannot allocate %zu bytes of workspace for %zu keys", bytes, nkeys);
   }
-  if (fr_nodes > b->cap_fr) {
-    size_t c1 = b->cap_fr, c2 = b->cap_fr;
-    if (int rc = grow_dev(b->d_fr_seed, c1, fr_nodes, "frontier seeds")) return rc;
-    if (int rc = grow_dev(b->d_fr_t, c2, fr_nodes, "frontier control bits")) return rc;
-    b->cap_fr = fr_nodes;
+  auto dev = [&](size_t at) { return static_cast<uint8_t*>(b->d_arena) + at; };
+  auto host = [&](size_t at) { return static_cast<uint8_t*>(b->h_arena) + at; };
+  b->d_keys = reinterpret_cast<KeyDev*>(dev(keys_at));
+  b->h_keys = reinterpret_cast<KeyDev*>(host(keys_at));
+  b->d_out = reinterpret_cast<uint4*>(dev(out_at));
+  b->h_out = host(out_at);
+  b->d_partial = reinterpret_cast<uint4*>(dev(partial_at));
+  b->d_fr_seed = reinterpret_cast<uint4*>(dev(fr_at));
+  b->d_fr_t = dev(fr_t_at);
+  for (int i = 0; i < 2; ++i) {
+    b->d_tmp_seed[i] = reinterpret_cast<uint4*>(dev(tmp_at[i]));
+    b->d_tmp_t[i] = dev(tmp_t_at[i]);
   }
-  if (tmp_nodes > b->cap_tmp) {
-    for (int i = 0; i < 2; ++i) {
-      size_t c1 = b->cap_tmp, c2 = b->cap_tmp;
-      if (int rc = grow_dev(b->d_tmp_seed[i], c1, tmp_nodes, "frontier chain")) return rc;
-      if (int rc = grow_dev(b->d_tmp_t[i], c2, tmp_nodes, "frontier chain")) return rc;
-    }
-    b->cap_tmp = tmp_nodes;
-  }
+  b->cap_keys = nkeys;
+  b->cap_partial = partial_u4;
+  b->cap_out = out_u4;
+  b->cap_fr = fr_nodes;
+  b->cap_tmp = tmp_nodes;
   return MG_OK;
 }
 
@@ -746,19 +750,10 @@ int mg_batch_destroy(mg_batch* b) {
   if (b->stream) cudaStreamSynchronize(b->stream);
   if (b->gexec) cudaGraphExecDestroy(b->gexec);
   if (b->gexec_io) cudaGraphExecDestroy(b->gexec_io);
-  if (b->d_keys) cudaFree(b->d_keys);
-  if (b->h_keys) cudaFreeHost(b->h_keys);
-  if (b->d_partial) cudaFree(b->d_partial);
-  if (b->d_out) cudaFree(b->d_out);
-  if (b->h_out) cudaFreeHost(b->h_out);
+  if (b->d_arena) cudaFree(b->d_arena);
+  if (b->h_arena) cudaFreeHost(b->h_arena);
   if (b->d_jobs) cudaFree(b->d_jobs);
   if (b->h_jobs) cudaFreeHost(b->h_jobs);
-  if (b->d_fr_seed) cudaFree(b->d_fr_seed);
-  if (b->d_fr_t) cudaFree(b->d_fr_t);
-  for (int i = 0; i < 2; ++i) {
-    if (b->d_tmp_seed[i]) cudaFree(b->d_tmp_seed[i]);
-    if (b->d_tmp_t[i]) cudaFree(b->d_tmp_t[i]);
-  }
   for (cudaEvent_t e : {b->ev_k0, b->ev_km, b->ev_k1, b->ev_done, b->ev_h0, b->ev_h1})
     if (e) cudaEventDestroy(e);
   if (b->stream) cudaStreamDestroy(b->stream);
