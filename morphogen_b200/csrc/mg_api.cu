@@ -308,6 +308,10 @@ int grow(mg_batch* b, size_t nkeys, size_t partial_u4, size_t out_u4, size_t fr_
   out_u4 = std::max(out_u4, b->cap_out);
   fr_nodes = std::max(fr_nodes, b->cap_fr);
   tmp_nodes = std::max(tmp_nodes, b->cap_tmp);
+  b->planned = false;  // the old plan's pointers go with the old allocation
+  b->d_keys = b->h_keys = nullptr;
+  b->d_out = b->d_partial = b->d_fr_seed = nullptr;
+  b->h_out = b->d_fr_t = nullptr;
   if (b->d_arena) cudaFree(b->d_arena);
   if (b->h_arena) cudaFreeHost(b->h_arena);
   b->d_arena = nullptr;
