@@ -1083,7 +1083,7 @@ int plan_warp(mg_batch* b, const std::vector<SegPlan>& segs, int G, uint32_t VT,
   // 2^20 x 256 B pass on 16 warps then take 8 item times of a scheduler
   // instead of 7: 145 us against 137).  With many, one queue evens out the
   // warps' drift (2^25 x 32 B: 2.54 ms against 2.57).
-  L.w.queues = items <= (uint64_t)4 * L.NW * ctx->sms ? 4u : 1u;
+  L.w.queues = items <= (uint64_t)4 * L.NW * ctx->sms ? std::min(4u, L.NW) : 1u;
   if (int rc = prepare_warp(ctx, G, VT, L.smem)) return rc;
   const int occ = mg::warp_occupancy(G, VT, L.smem, L.NW);
   if (occ <= 0) return fail(MG_EINVAL, "warp kernel does not fit the device");

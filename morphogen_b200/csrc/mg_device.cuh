@@ -364,7 +364,7 @@ struct WarpScanParams {
   uint32_t cols;
   uint32_t V;           // uint4 per row of every segment of the launch
   uint32_t slots;       // stack levels per lane and key
-  uint32_t queues;      // item queues per CTA: 1, or 4 (one per warp scheduler)
+  uint32_t queues;      // item queues per CTA: 1, or one per warp scheduler (up to 4, at most the CTA's warps)
 };
 
 // A key whose table has a pending delta: its key slot, its first share column

@@ -510,23 +510,26 @@ __device__ __forceinline__ void copy_async(uint4* dst, const uint4* src) {
 }
 
 // The items of a CTA's contiguous range, taken one at a time by its warps: from
-// one queue, or from four, each a quarter of the range and served by the warps
-// of one scheduler (warp w issues on scheduler w mod 4).  See WarpScanParams.
+// one queue, or from four, each served by the warps of one scheduler (warp w
+// issues on scheduler w mod 4) and holding every fourth item, so that a CTA of
+// as many warps as items has one for each (contiguous quarters gave some queues
+// more items than warps: 175056 x 256 B with 3 keys 44.5 us against 50.8, 60000
+// x 32 B 31.4 against 34.2, 20000 x 256 B with 24 keys 43.4 against 50.8).  The
+// step is read from the launch parameters: in a register it cost the pair scan
+// 0.4% (2^22 x 32 B: 349.6 us against 347.9).  See WarpScanParams.
 struct ItemQueue {
-  uint64_t begin, end;
+  uint64_t first, end;
   uint32_t* next;
-  __device__ __forceinline__ ItemQueue(const WarpScanParams& p, uint32_t* s_next, uint32_t warp, uint32_t nw) {
-    const uint32_t nq = nw < p.queues ? nw : p.queues, q = warp % nq;
-    const uint64_t b = (uint64_t)blockIdx.x * p.items / gridDim.x;
-    const uint64_t n = (uint64_t)(blockIdx.x + 1) * p.items / gridDim.x - b;
-    begin = b + n * q / nq;
-    end = b + n * (q + 1) / nq;
+  __device__ __forceinline__ ItemQueue(const WarpScanParams& p, uint32_t* s_next, uint32_t warp) {
+    const uint32_t q = warp % p.queues;
+    first = (uint64_t)blockIdx.x * p.items / gridDim.x + q;
+    end = (uint64_t)(blockIdx.x + 1) * p.items / gridDim.x;
     next = s_next + q;
   }
-  __device__ __forceinline__ bool take(const uint32_t lane, uint64_t& item) const {
+  __device__ __forceinline__ bool take(const WarpScanParams& p, const uint32_t lane, uint64_t& item) const {
     uint32_t rel = 0;
-    if (lane == 0) rel = atomicAdd(next, 1u);
-    item = begin + __shfl_sync(0xFFFFFFFFu, rel, 0);
+    if (lane == 0) rel = atomicAdd(next, p.queues);
+    item = first + __shfl_sync(0xFFFFFFFFu, rel, 0);
     return item < end;
   }
 };
@@ -575,7 +578,7 @@ __global__ void __launch_bounds__(warp_cta_warps(1) * 32, 1) scan_pair_kernel(co
   const LaneStack st = {stk4 + (size_t)warp * p.slots * 32 + lane,
                         reinterpret_cast<int8_t*>(stk4 + (size_t)nw * p.slots * 32) + (size_t)warp * p.slots * 32 + lane};
   uint4* const my_partial = p.partial + ((uint64_t)blockIdx.x * nw + warp) * p.cols;
-  const ItemQueue queue(p, s_next, warp, nw);
+  const ItemQueue queue(p, s_next, warp);
   if (threadIdx.x < 4) s_next[threadIdx.x] = 0;
   __syncthreads();
   chain_begin();
@@ -600,7 +603,7 @@ __global__ void __launch_bounds__(warp_cta_warps(1) * 32, 1) scan_pair_kernel(co
     }
   };
 
-  for (uint64_t item; queue.take(lane, item);) {
+  for (uint64_t item; queue.take(p, lane, item);) {
     uint32_t si = 0;
     while (si + 1 < p.nsegs && item >= p.seg[si + 1].item_begin) ++si;
     const WarpSeg& sg = p.seg[si];
@@ -718,7 +721,7 @@ __global__ void __launch_bounds__(warp_cta_warps(G) * 32, 1)
 
   uint4* const my_partial = p.partial + ((uint64_t)blockIdx.x * nw + warp) * p.cols;
   for (uint32_t c = lane; c < p.cols; c += 32) my_partial[c] = make_uint4(0u, 0u, 0u, 0u);
-  const ItemQueue queue(p, s_next, warp, nw);
+  const ItemQueue queue(p, s_next, warp);
   if (threadIdx.x < 4) s_next[threadIdx.x] = 0;
   __syncthreads();
 
@@ -813,7 +816,7 @@ __global__ void __launch_bounds__(warp_cta_warps(G) * 32, 1)
     }
   };
 
-  for (uint64_t item; queue.take(lane, item);) {
+  for (uint64_t item; queue.take(p, lane, item);) {
     uint32_t si = 0;
     while (si + 1 < p.nsegs && item >= p.seg[si + 1].item_begin) ++si;
     const WarpSeg& sg = p.seg[si];

@@ -36,6 +36,33 @@ def test_own_rows_cta_widths(scanner, oracle_mod, row_bytes, M, items):
     db.close()
 
 
+@pytest.mark.parametrize("row_bytes", [32, 48, 256])
+@pytest.mark.parametrize("per_cta,extra", [(2, 1), (5, -1), (6, 0), (12, 5), (80, 0), (80, 1)])
+def test_scheduler_queues_cover_every_item(scanner, oracle_mod, row_bytes, per_cta, extra):
+    # Items that do not divide into four queues, and both sides of the line
+    # (80 per CTA of 20 warps, 64 of 16) where the CTAs go over to one queue.
+    G_ = 1 if row_bytes == 32 else 3
+    per_cta = 64 if per_cta == 80 and G_ == 3 else per_cta
+    sms = scanner.device_info()["sm_count"]
+    items = per_cta * sms + extra
+    nrows = items * 64 - 5
+    d = max(7, (nrows - 1).bit_length())
+    db = G.GpuPageMatrix.from_seed(scanner, nrows, row_bytes, seed=items)
+    host = oracle_mod.fill_splitmix(0, nrows * row_bytes, items).reshape(nrows, row_bytes)
+    keys = [oracle_keypair(oracle_mod, d, (nrows - 1) // (j + 1), seed=97, i=items + j)[0] for j in range(G_)]
+    ws = scanner.workspace()
+    ws.set_shape(6, G_)
+    ws.set_keys([db] * G_, keys)
+    plan = ws.plan()
+    assert plan["items"] == items and plan["grid"] <= sms
+    want = oracle_mod.scan_fused(keys, host, row_bytes)
+    for graph in (False, True):
+        ws.launch(graph=graph)
+        assert ws.read() == want
+    ws.close()
+    db.close()
+
+
 @pytest.mark.parametrize("row_bytes", [48, 80, 112, 128, 192, 256, 272, 496, 512])
 @pytest.mark.parametrize("M,keys_per_item,nkeys", [(1, 3, 4), (2, 3, 3), (3, 3, 7), (4, 1, 2), (5, 2, 3), (9, 3, 3)])
 def test_block_scan_shapes(scanner, oracle_mod, row_bytes, M, keys_per_item, nkeys):
