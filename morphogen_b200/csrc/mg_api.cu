@@ -1094,8 +1094,10 @@ int plan_warp(mg_batch* b, const std::vector<SegPlan>& segs, int G, uint32_t VT,
   // that two never share one.  The CTAs arrive while the frontier still runs
   // and narrow ones packed onto the SMs it left free (3 keys: 140000 x 128 B
   // 38.8 us against 47.2, 60000 x 128 B 32.7 against 35.2, 30000 x 128 B 26.3
-  // against 28.2; wide CTAs unchanged).
-  if (L.grid <= (uint32_t)ctx->sms) {
+  // against 28.2; 12000 x 128 B, two warps a CTA, 24.9 against 28.9; wide CTAs
+  // unchanged).  CTAs of one warp gain nothing from it (4099 x 32 B 25.8 against
+  // 25.2, 2774 x 96 B 23.4 against 22.8) and keep their size.
+  if (L.NW > 1 && L.grid <= (uint32_t)ctx->sms) {
     const size_t pad = std::min(ctx->smem_optin, ctx->smem_optin / 2 + 2048);
     if (L.smem < pad) {
       L.smem = pad;
