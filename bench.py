@@ -553,9 +553,10 @@ def rooflines(bytes_scanned: int, nodes: int, seconds: float, prg_peak: float, h
 
 def traffic_for(traffic_rec: dict, kernel_kind: int, bytes_scanned: int, row_bytes: int = 32):
     """DRAM read + write bytes per launch: the ratio ncu measured on a smaller
-    capture of the same kernel (the warp kernel's own-rows and wide-row
-    instantiations apart), scaled by the rows scanned."""
-    name = "scan_kernel" if kernel_kind != 2 else ("scan_warp_kernel" if row_bytes <= 32 else "scan_warp_kernel_wide")
+    capture of the same kernel (of the warp kernels the pair scan and the block
+    scan apart), scaled by the rows scanned."""
+    name = "scan_kernel" if kernel_kind != 2 else ("scan_pair_kernel" if row_bytes in (16, 32, 64)
+                                                   else "scan_block_kernel")
     rec = traffic_rec.get(name, {})
     if not rec.get("table_bytes"):
         return None

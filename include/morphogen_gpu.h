@@ -66,7 +66,8 @@ typedef struct {
 /* Scan kernels.  CTA: a CTA expands a 2^S-row tile (breadth-first in shared
  * memory, then one depth-first walk per thread); any row size.  WARP: a
  * frontier of tree nodes is computed breadth-first up front and every warp
- * walks 32 x 2^M rows on its own; rows of 16..512 B (power of two). */
+ * walks 32 x 2^M rows on its own; rows of 16..512 B (pinning it needs a power
+ * of two). */
 enum { MG_KERNEL_AUTO = 0, MG_KERNEL_CTA = 1, MG_KERNEL_WARP = 2 };
 
 /* Launch shape chosen for a pass (first launch; subtree_bits over all). */
