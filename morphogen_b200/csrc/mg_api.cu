@@ -299,24 +299,27 @@ int prepare_warp(mg_context* ctx, int G, uint32_t VT, size_t smem) {
 // allocation, both pinned ones parts of another, because the first pass of a
 // workspace pays for each call of cudaMalloc (about 0.1 ms; five to nine of
 // them took 0.4 of the 0.7 ms of a first call over 1000003 x 48 B).
-int grow(mg_batch* b, size_t nkeys, size_t partial_u4, size_t out_u4, size_t fr_nodes, size_t tmp_nodes) {
-  if (nkeys <= b->cap_keys && partial_u4 <= b->cap_partial && out_u4 <= b->cap_out && fr_nodes <= b->cap_fr &&
-      tmp_nodes <= b->cap_tmp)
+int grow(mg_batch* b, size_t nkeys, size_t njobs, size_t partial_u4, size_t out_u4, size_t fr_nodes,
+         size_t tmp_nodes) {
+  if (nkeys <= b->cap_keys && njobs <= b->cap_jobs && partial_u4 <= b->cap_partial && out_u4 <= b->cap_out &&
+      fr_nodes <= b->cap_fr && tmp_nodes <= b->cap_tmp)
     return MG_OK;
   nkeys = std::max(nkeys, b->cap_keys);
+  njobs = std::max(njobs, b->cap_jobs);
   partial_u4 = std::max(partial_u4, b->cap_partial);
   out_u4 = std::max(out_u4, b->cap_out);
   fr_nodes = std::max(fr_nodes, b->cap_fr);
   tmp_nodes = std::max(tmp_nodes, b->cap_tmp);
   b->planned = false;  // the old plan's pointers go with the old allocation
   b->d_keys = b->h_keys = nullptr;
+  b->d_jobs = b->h_jobs = nullptr;
   b->d_out = b->d_partial = b->d_fr_seed = nullptr;
   b->h_out = b->d_fr_t = nullptr;
   if (b->d_arena) cudaFree(b->d_arena);
   if (b->h_arena) cudaFreeHost(b->h_arena);
   b->d_arena = nullptr;
   b->h_arena = nullptr;
-  b->cap_keys = b->cap_partial = b->cap_out = b->cap_fr = b->cap_tmp = 0;
+  b->cap_keys = b->cap_jobs = b->cap_partial = b->cap_out = b->cap_fr = b->cap_tmp = 0;
   size_t bytes = 0;
   auto part = [&](size_t n) {
     const size_t at = bytes;
@@ -325,7 +328,7 @@ int grow(mg_batch* b, size_t nkeys, size_t partial_u4, size_t out_u4, size_t fr_
   };
   // Keys, then their warp-kernel constants (KeyAux) right after the pass's keys.
   const size_t key_bytes = nkeys * (sizeof(KeyDev) + sizeof(mg::KeyAux));
-  const size_t keys_at = part(key_bytes), out_at = part(out_u4 * 16);
+  const size_t keys_at = part(key_bytes), out_at = part(out_u4 * 16), jobs_at = part(njobs * sizeof(mg::DeltaJob));
   const size_t host_bytes = bytes;
   const size_t partial_at = part(partial_u4 * 16), fr_at = part(fr_nodes * 16), fr_t_at = part(fr_nodes);
   size_t tmp_at[2], tmp_t_at[2];
@@ -338,6 +341,7 @@ int grow(mg_batch* b, size_t nkeys, size_t partial_u4, size_t out_u4, size_t fr_
     if (b->d_arena) cudaFree(b->d_arena);
     b->d_arena = nullptr;
     b->h_arena = nullptr;
+    b->launched = false;  // the last pass's shares are gone too
     return fail(MG_ENOMEM, "cannot allocate %zu bytes of workspace for %zu keys", bytes, nkeys);
   }
   auto dev = [&](size_t at) { return static_cast<uint8_t*>(b->d_arena) + at; };
@@ -346,6 +350,8 @@ int grow(mg_batch* b, size_t nkeys, size_t partial_u4, size_t out_u4, size_t fr_
   b->h_keys = reinterpret_cast<KeyDev*>(host(keys_at));
   b->d_out = reinterpret_cast<uint4*>(dev(out_at));
   b->h_out = host(out_at);
+  b->d_jobs = reinterpret_cast<mg::DeltaJob*>(dev(jobs_at));
+  b->h_jobs = reinterpret_cast<mg::DeltaJob*>(host(jobs_at));
   b->d_partial = reinterpret_cast<uint4*>(dev(partial_at));
   b->d_fr_seed = reinterpret_cast<uint4*>(dev(fr_at));
   b->d_fr_t = dev(fr_t_at);
@@ -354,6 +360,7 @@ int grow(mg_batch* b, size_t nkeys, size_t partial_u4, size_t out_u4, size_t fr_
     b->d_tmp_t[i] = dev(tmp_t_at[i]);
   }
   b->cap_keys = nkeys;
+  b->cap_jobs = njobs;
   b->cap_partial = partial_u4;
   b->cap_out = out_u4;
   b->cap_fr = fr_nodes;
@@ -756,8 +763,6 @@ int mg_batch_destroy(mg_batch* b) {
   if (b->gexec_io) cudaGraphExecDestroy(b->gexec_io);
   if (b->d_arena) cudaFree(b->d_arena);
   if (b->h_arena) cudaFreeHost(b->h_arena);
-  if (b->d_jobs) cudaFree(b->d_jobs);
-  if (b->h_jobs) cudaFreeHost(b->h_jobs);
   for (cudaEvent_t e : {b->ev_k0, b->ev_km, b->ev_k1, b->ev_done, b->ev_h0, b->ev_h1})
     if (e) cudaEventDestroy(e);
   if (b->stream) cudaStreamDestroy(b->stream);
@@ -1287,28 +1292,15 @@ int plan_pass(mg_batch* b) {
       if (b->in_tables[i] == dl.table) jobs.push_back(delta_job(launches, dl.table, key_slot[i], key_col[i]));
     dl.njobs = (uint32_t)jobs.size() - dl.job0;
   }
-  if (jobs.size() > b->cap_jobs) {
-    if (b->d_jobs) cudaFree(b->d_jobs);
-    if (b->h_jobs) cudaFreeHost(b->h_jobs);
-    b->d_jobs = nullptr;
-    b->h_jobs = nullptr;
-    b->cap_jobs = 0;
-    if (cudaMalloc(&b->d_jobs, jobs.size() * sizeof(mg::DeltaJob)) != cudaSuccess ||
-        cudaMallocHost(&b->h_jobs, jobs.size() * sizeof(mg::DeltaJob)) != cudaSuccess) {
-      cudaGetLastError();
-      return fail(MG_ENOMEM, "cannot allocate delta job lists");
-    }
-    b->cap_jobs = jobs.size();
-  }
+
+  size_t max_partial = 0;
+  for (const mg_batch::Launch& L : launches) max_partial = std::max(max_partial, (size_t)L.nparts * L.cols);
+  if (int rc = grow(b, nkeys, jobs.size(), max_partial, total_cols, (size_t)fr_cursor, tmp_need)) return rc;
   if (!jobs.empty()) {
     std::memcpy(b->h_jobs, jobs.data(), jobs.size() * sizeof(mg::DeltaJob));
     MG_CUDA(cudaMemcpyAsync(b->d_jobs, b->h_jobs, jobs.size() * sizeof(mg::DeltaJob), cudaMemcpyHostToDevice, b->stream));
   }
   b->deltas = std::move(deltas);
-
-  size_t max_partial = 0;
-  for (const mg_batch::Launch& L : launches) max_partial = std::max(max_partial, (size_t)L.nparts * L.cols);
-  if (int rc = grow(b, nkeys, max_partial, total_cols, (size_t)fr_cursor, tmp_need)) return rc;
   mg::KeyAux* const h_aux = reinterpret_cast<mg::KeyAux*>(b->h_keys + nkeys);
   const mg::KeyAux* const d_aux = reinterpret_cast<const mg::KeyAux*>(b->d_keys + nkeys);
   for (uint32_t i = 0; i < nkeys; ++i) {
@@ -1649,6 +1641,7 @@ std::vector<uint8_t> pass_signature(const mg_batch* b) {
     add(&dl.table->delta_cap, sizeof dl.table->delta_cap);
   }
   add(&b->d_out, sizeof b->d_out);
+  add(&b->d_jobs, sizeof b->d_jobs);
   add(&b->d_fr_seed, sizeof b->d_fr_seed);
   return sig;
 }

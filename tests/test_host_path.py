@@ -1,0 +1,90 @@
+"""Host path of the library on a CPU (see fake_device.py): workspaces, graph
+reuse, planning and memory limits.  Nothing is computed here; what is checked
+is which memory a launch is given, and which calls are taken or refused."""
+import ctypes as C
+
+import pytest
+
+import fake_device
+from morphogen_b200 import _native as N
+from morphogen_b200 import gpu_dpf as G
+
+
+@pytest.fixture(scope="module")
+def fake_path():
+    return fake_device.build()
+
+
+@pytest.fixture
+def fake(fake_path):
+    with fake_device.fake_library(fake_path) as L:
+        L.fake_reset(178 * fake_device.GIB, 0)
+        yield L
+
+
+@pytest.fixture
+def fscanner(fake):
+    s = G.GpuScanner(0)
+    yield s
+    s.close()
+
+
+def key(d, target=0):
+    return G.generate_chacha_dpf_keys(G.ChaChaParams(d), target)[0].to_bytes()
+
+
+def delta_args(L):
+    """Job list, entry indices, entry rows and count of the last delta launch."""
+    out = (C.c_uint64 * 4)()
+    L.fake_last_delta(out)
+    return tuple(out)
+
+
+def test_replayed_graphs_never_read_a_freed_job_list(fake, fscanner):
+    # 24 keys size the workspace before the table has a delta buffer; with one,
+    # 3 keys are captured, 24 keys need a longer job list, and the 3 keys' next
+    # replay must not use the first list.
+    t = G.GpuPageMatrix.alloc_empty(fscanner, 70_001, 32)
+    keys = [key(17, i) for i in range(24)]
+    fscanner.scan_keys(t, keys)
+    t.delta_reserve(100)
+    for n in (3, 3, 24, 3, 3, 24, 24, 3, 3):
+        fscanner.scan_keys(t, keys[:n])
+        assert fake.fake_dead_launches() == 0, f"{n} keys"
+    ws = fscanner.workspace()
+    ws.set_keys([t] * 3, keys[:3])
+    ws.launch(graph=True)
+    for n in (24, 3):
+        ws.set_keys([t] * n, keys[:n])
+    ws.launch(graph=True)
+    graph = delta_args(fake)
+    ws.launch()
+    assert graph == delta_args(fake) and fake.fake_dead_launches() == 0
+    ws.close()
+    t.close()
+
+
+@pytest.mark.parametrize("fails", [1 << i for i in range(4)])
+def test_a_failed_growth_leaves_nothing_launchable(fake, fscanner, fails):
+    t = G.GpuPageMatrix.alloc_empty(fscanner, 5000, 32)
+    t.delta_reserve(10)
+    keys = [key(13, i) for i in range(40)]
+    ws = fscanner.workspace()
+    ws.set_keys([t] * 2, keys[:2])
+    ws.launch()
+    fake.fake_fail(fails)
+    try:
+        ws.set_keys([t] * 40, keys)
+    except N.MgError as e:
+        assert e.code == N.MG_ENOMEM
+        for call in (ws.launch, lambda: ws.launch(graph=True), ws.plan, ws.read):
+            with pytest.raises(N.MgError) as err:
+                call()
+            assert err.value.code == N.MG_EINVAL
+    fake.fake_fail(0)
+    ws.set_keys([t] * 40, keys)
+    ws.launch()
+    ws.launch(graph=True)
+    assert len(ws.read()) == 40 and fake.fake_dead_launches() == 0
+    ws.close()
+    t.close()
