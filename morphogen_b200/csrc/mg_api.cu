@@ -258,7 +258,7 @@ struct mg_batch {
   std::vector<uint32_t> plan_slot;     // input key i -> key slot
   std::vector<uint32_t> plan_depth;    // input key i -> domain bits
   std::vector<const mg_table*> plan_tables;
-  std::vector<std::pair<const void*, uint32_t>> plan_deltas;  // per input key: delta buffer, capacity
+  std::vector<std::array<uint64_t, 4>> plan_deltas;  // per input key: its table's delta buffer (delta_shape)
   std::vector<std::array<uint64_t, 4>> plan_shapes;  // per input key: table memory, rows, row bytes, first row
   int plan_kind = -1;
   uint32_t plan_S = 0, plan_G = 0;
@@ -271,6 +271,13 @@ namespace {
 // address can come back for a different table).
 std::array<uint64_t, 4> table_shape(const mg_table* t) {
   return {(uint64_t)(uintptr_t)t->d, t->rows, t->row_bytes, t->first};
+}
+
+// A table's delta buffer as the delta kernel is given it.  Each of its arrays
+// may move by itself: one may get an address back that another does not.
+std::array<uint64_t, 4> delta_shape(const mg_table* t) {
+  return {(uint64_t)(uintptr_t)t->d_delta_idx, (uint64_t)(uintptr_t)t->d_delta_diff,
+          (uint64_t)(uintptr_t)t->d_delta_count, t->delta_cap};
 }
 
 
@@ -1337,7 +1344,7 @@ int plan_pass(mg_batch* b) {
   b->plan_deltas.resize(nkeys);
   for (uint32_t i = 0; i < nkeys; ++i) {
     b->plan_depth[i] = parsed[i].domain_bits;
-    b->plan_deltas[i] = {b->in_tables[i]->d_delta_idx, b->in_tables[i]->delta_cap};
+    b->plan_deltas[i] = delta_shape(b->in_tables[i]);
   }
   b->plan_tables = b->in_tables;
   b->plan_shapes.resize(nkeys);
@@ -1423,7 +1430,7 @@ int mg_batch_set_keys(mg_batch* b, const mg_table* const* tables, const uint8_t*
     bool same = true;
     for (uint32_t i = 0; i < nkeys && same; ++i)
       same = parsed[i].domain_bits == b->plan_depth[i] && b->plan_shapes[i] == table_shape(tabs[i]) &&
-             b->plan_deltas[i] == std::make_pair((const void*)tabs[i]->d_delta_idx, tabs[i]->delta_cap);
+             b->plan_deltas[i] == delta_shape(tabs[i]);
     int kind = b->kind_pref;
     uint32_t S = b->shape_S, G = b->shape_G;
     if (same && kind == MG_KERNEL_AUTO && S == 0 && G == 0) {
@@ -1637,8 +1644,8 @@ std::vector<uint8_t> pass_signature(const mg_batch* b) {
   }
   for (const mg_batch::DeltaLaunch& dl : b->deltas) {
     add(&dl, sizeof dl);
-    add(&dl.table->d_delta_idx, sizeof dl.table->d_delta_idx);
-    add(&dl.table->delta_cap, sizeof dl.table->delta_cap);
+    const std::array<uint64_t, 4> shape = delta_shape(dl.table);
+    add(&shape, sizeof shape);
   }
   add(&b->d_out, sizeof b->d_out);
   add(&b->d_jobs, sizeof b->d_jobs);

@@ -88,3 +88,38 @@ def test_a_failed_growth_leaves_nothing_launchable(fake, fscanner, fails):
     assert len(ws.read()) == 40 and fake.fake_dead_launches() == 0
     ws.close()
     t.close()
+
+
+@pytest.mark.parametrize("call", ["scan", "workspace"])
+def test_graphs_follow_a_delta_buffer_that_keeps_its_index_address(fake, fscanner, call):
+    # A buffer of 8, 16, then 8 entries again: the index array gets its first
+    # address back, the row array, whose memory a table took meanwhile, does not.
+    fake.fake_reset(178 * fake_device.GIB, 1)
+    t = G.GpuPageMatrix.alloc_empty(fscanner, 5000, 48)
+    ws = fscanner.workspace()
+    keys = [key(13, i) for i in range(3)]
+
+    def run():
+        if call == "scan":
+            for _ in range(3):
+                fscanner.scan_keys(t, keys)
+        else:
+            ws.set_keys([t] * 3, keys)
+            ws.launch(graph=True)
+        replayed = delta_args(fake)
+        ws.set_keys([t] * 3, keys)
+        ws.launch()
+        return replayed[1:], delta_args(fake)[1:]
+
+    t.delta_reserve(8)
+    first, direct = run()
+    assert first == direct
+    t.delta_reserve(16)
+    other = G.GpuPageMatrix.alloc_empty(fscanner, 8, 48)
+    t.delta_reserve(8)
+    again, direct = run()
+    assert direct[0] == first[0] and direct[1] != first[1]
+    assert again == direct and fake.fake_dead_launches() == 0
+    ws.close()
+    other.close()
+    t.close()
