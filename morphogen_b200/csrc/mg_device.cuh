@@ -197,15 +197,17 @@ __device__ __forceinline__ uint4 leaf_mask(const uint4 s, const uint32_t t, cons
   return make_uint4(s.x ^ (f.x & m), s.y ^ (f.y & m), s.z ^ (f.z & m), s.w ^ (f.w & m));
 }
 
-// Same as expand_cw with the key read through the read-only data path (the
-// key is uniform across a warp, so every load is a broadcast L1 hit).
+// Same as expand_cw with the key in global memory (it is uniform across a
+// warp, so every load is a broadcast L1 hit).  Keys and their constants are
+// read with plain loads: the pass's first kernel writes them, and a kernel of
+// the pass may have been launched before that one has ended.
 template <bool FMA = true>
-__device__ __forceinline__ void expand_cw_g(const uint4 s, const uint32_t t, const KeyDev* __restrict__ k,
+__device__ __forceinline__ void expand_cw_g(const uint4 s, const uint32_t t, const KeyDev* k,
                                             const uint32_t level, uint4& L, uint32_t& tl, uint4& R,
                                             uint32_t& tr) {
-  const uint4 cw = __ldg(&k->cw_seed[level]);
-  const uint32_t cwl = __ldg(&k->cw_tl[level]);
-  const uint32_t cwr = __ldg(&k->cw_tr[level]);
+  const uint4 cw = k->cw_seed[level];
+  const uint32_t cwl = k->cw_tl[level];
+  const uint32_t cwr = k->cw_tr[level];
   prg_expand<FMA>(s, L, R, tl, tr);
   const uint32_t m = (t == 1u) ? 0xFFFFFFFFu : 0u;
   L.x ^= cw.x & m; L.y ^= cw.y & m; L.z ^= cw.z & m; L.w ^= cw.w & m;
@@ -214,9 +216,9 @@ __device__ __forceinline__ void expand_cw_g(const uint4 s, const uint32_t t, con
   tr ^= cwr & m;
 }
 
-__device__ __forceinline__ uint4 leaf_mask_g(const uint4 s, const uint32_t t, const KeyDev* __restrict__ k) {
+__device__ __forceinline__ uint4 leaf_mask_g(const uint4 s, const uint32_t t, const KeyDev* k) {
   const uint32_t m = (t == 1u) ? 0xFFFFFFFFu : 0u;
-  const uint4 f = __ldg(&k->final_cw);
+  const uint4 f = k->final_cw;
   return make_uint4(s.x ^ (f.x & m), s.y ^ (f.y & m), s.z ^ (f.z & m), s.w ^ (f.w & m));
 }
 
@@ -224,10 +226,10 @@ __device__ __forceinline__ uint4 leaf_mask_g(const uint4 s, const uint32_t t, co
 // (seeds L, R, bits bl, br), with t carried as a mask (KeyAux): m is all ones
 // iff the parent's t == 1; ml / mr are the children's masks.
 __device__ __forceinline__ void apply_cw_m(uint4& L, uint4& R, const uint32_t bl, const uint32_t br, const uint32_t m,
-                                           const KeyDev* __restrict__ k, const KeyAux* __restrict__ a,
+                                           const KeyDev* k, const KeyAux* a,
                                            const uint32_t level, uint32_t& ml, uint32_t& mr) {
-  const uint4 cw = __ldg(&k->cw_seed[level]);
-  const uint4 tm = __ldg(&a->cw_tm[level]);
+  const uint4 cw = k->cw_seed[level];
+  const uint4 tm = a->cw_tm[level];
   L.x ^= cw.x & m; L.y ^= cw.y & m; L.z ^= cw.z & m; L.w ^= cw.w & m;
   R.x ^= cw.x & m; R.y ^= cw.y & m; R.z ^= cw.z & m; R.w ^= cw.w & m;
   ml = ((0u - bl) ^ (tm.x & m)) & ~(tm.y & m);
@@ -238,18 +240,18 @@ __device__ __forceinline__ void apply_cw_m(uint4& L, uint4& R, const uint32_t bl
 // seeds, with the level's correction word and the final correction word
 // folded into one table entry per child.
 __device__ __forceinline__ void leaf_terms_m(const uint4 L, const uint4 R, const uint32_t bl, const uint32_t br,
-                                             const uint32_t m, const KeyAux* __restrict__ a, uint4& mask_l,
+                                             const uint32_t m, const KeyAux* a, uint4& mask_l,
                                              uint4& mask_r) {
   const uint32_t p2 = m & 2u;  // 2 * parent bit
-  const uint4 cl = __ldg(&a->leaf[p2 | bl]);
-  const uint4 cr = __ldg(&a->leaf[4u + (p2 | br)]);
+  const uint4 cl = a->leaf[p2 | bl];
+  const uint4 cr = a->leaf[4u + (p2 | br)];
   mask_l = make_uint4(L.x ^ cl.x, L.y ^ cl.y, L.z ^ cl.z, L.w ^ cl.w);
   mask_r = make_uint4(R.x ^ cr.x, R.y ^ cr.y, R.z ^ cr.z, R.w ^ cr.w);
 }
 
 // One node expansion with the level's correction word, t carried as a mask.
-__device__ __forceinline__ void expand_cw_m(const uint4 s, const uint32_t m, const KeyDev* __restrict__ k,
-                                            const KeyAux* __restrict__ a, const uint32_t level, uint4& L,
+__device__ __forceinline__ void expand_cw_m(const uint4 s, const uint32_t m, const KeyDev* k,
+                                            const KeyAux* a, const uint32_t level, uint4& L,
                                             uint32_t& ml, uint4& R, uint32_t& mr) {
   uint32_t bl, br;
   prg_expand(s, L, R, bl, br);
@@ -257,7 +259,7 @@ __device__ __forceinline__ void expand_cw_m(const uint4 s, const uint32_t m, con
 }
 
 // The leaf pair below node s of level d - 1.
-__device__ __forceinline__ void leaf_pair_m(const uint4 s, const uint32_t m, const KeyAux* __restrict__ a,
+__device__ __forceinline__ void leaf_pair_m(const uint4 s, const uint32_t m, const KeyAux* a,
                                             uint4& mask_l, uint4& mask_r) {
   uint4 L, R;
   uint32_t bl, br;

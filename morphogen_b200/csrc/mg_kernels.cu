@@ -38,7 +38,12 @@ namespace mg {
 // Every kernel of a pass begins with this: it lets the pass's next kernel be
 // launched while this one runs (its CTAs take their places as these leave) and
 // then waits until the kernel before it has completed and its writes are
-// visible.  Nothing in global memory is touched earlier.  See launch_chained.
+// visible.  Nothing in global memory is touched earlier, and what a kernel of
+// the pass writes (keys, frontier, partial rows, shares) or the host may write
+// beside it (a delta buffer) is read with plain loads: the read-only path and
+// __restrict__ promise data that nothing writes while the kernel lives, and its
+// life now begins before that of its predecessors ends.  Only the table's rows,
+// which no kernel of a pass writes, are read through __ldg.  See launch_chained.
 __device__ __forceinline__ void chain_begin() {
   cudaTriggerProgrammaticLaunchCompletion();
   cudaGridDependencySynchronize();
@@ -302,7 +307,7 @@ __global__ void __launch_bounds__(kThreads) frontier_kernel(const __grid_constan
   const uint64_t a = f.in_first + node;  // level index of the CTA's node
   const uint64_t g_out0 = a << f.c;      // level index of its first descendant
   if (g_out0 + (1ull << f.c) <= f.out_first || g_out0 >= f.out_first + f.n_out) return;  // uniform per CTA
-  const KeyDev* __restrict__ K = f.keys + j;
+  const KeyDev* K = f.keys + j;
   const uint32_t walk = f.walk ? f.L_in : 0u;  // levels above the CTA's node
   const uint32_t top = f.L_in - walk;          // level of the first node expanded
   const uint32_t wide = f.c < kFrontierWide ? f.c : kFrontierWide;
@@ -311,13 +316,13 @@ __global__ void __launch_bounds__(kThreads) frontier_kernel(const __grid_constan
     // Correction words of the step's levels, and its root.
     const uint32_t lvl = top + tid;
     if (tid < walk + f.c) {
-      s_cw[tid] = __ldg(&K->cw_seed[lvl]);
-      s_cwt[0][tid] = __ldg(&K->cw_tl[lvl]);
-      s_cwt[1][tid] = __ldg(&K->cw_tr[lvl]);
+      s_cw[tid] = K->cw_seed[lvl];
+      s_cwt[0][tid] = K->cw_tl[lvl];
+      s_cwt[1][tid] = K->cw_tr[lvl];
     }
     if (tid == 0) {
-      sa[0] = top == 0 ? __ldg(&K->root_seed) : f.in_seed[j * f.n_in + node];
-      ta[0] = (uint8_t)(top == 0 ? __ldg(&K->root_t) : f.in_t[j * f.n_in + node]);
+      sa[0] = top == 0 ? K->root_seed : f.in_seed[j * f.n_in + node];
+      ta[0] = (uint8_t)(top == 0 ? K->root_t : f.in_t[j * f.n_in + node]);
     }
   }
   uint4* cs = sa; uint8_t* ct = ta;
@@ -480,7 +485,7 @@ struct LaneStack {
 // pi + 1: s0, m0 and s1, m1.  For pi == 0 the caller passes the root in s0, m0;
 // otherwise the path re-joins the stack at relative level M - ffs(pi).  The
 // right children it passes are pushed, the last one staying in registers.
-__device__ __forceinline__ void walk_to_pairs(const KeyDev* __restrict__ K, const KeyAux* __restrict__ A,
+__device__ __forceinline__ void walk_to_pairs(const KeyDev* K, const KeyAux* A,
                                               const LaneStack st, const uint32_t pi, const uint32_t M,
                                               const uint32_t F, uint4& s0, uint32_t& m0, uint4& s1, uint32_t& m1) {
   uint32_t lvl = 0;
@@ -618,8 +623,8 @@ __global__ void __launch_bounds__(warp_cta_warps(1) * 32, 1) scan_pair_kernel(co
     const uint32_t M = sg.M, F = sg.d - M;
     const uint64_t node = (uint64_t)tile * 32 + lane;
     const bool valid = node < sg.nF;
-    const KeyDev* __restrict__ K = p.keys + sg.key_base + group;
-    const KeyAux* __restrict__ A = p.aux + sg.key_base + group;
+    const KeyDev* K = p.keys + sg.key_base + group;
+    const KeyAux* A = p.aux + sg.key_base + group;
     const uint64_t idx = sg.fr_base + (uint64_t)group * sg.nF + node;
     uint4 s0 = valid ? p.fr_seed[idx] : make_uint4(0u, 0u, 0u, 0u);
     uint32_t m0 = (valid && p.fr_t[idx] == 1) ? 0xFFFFFFFFu : 0u;
@@ -843,8 +848,8 @@ __global__ void __launch_bounds__(warp_cta_warps(G) * 32, 1)
     const uint32_t F = sg.d - M;
     const uint64_t node = (uint64_t)tile * 32 + lane;
     const bool valid = node < sg.nF;
-    const KeyDev* __restrict__ kp = p.keys + sg.key_base + (size_t)group * g;
-    const KeyAux* __restrict__ ap = p.aux + sg.key_base + (size_t)group * g;
+    const KeyDev* kp = p.keys + sg.key_base + (size_t)group * g;
+    const KeyAux* ap = p.aux + sg.key_base + (size_t)group * g;
     // A key's root waits in its stack's first slot, which level 1 takes over
     // once the walk has read it.
     for (uint32_t k = 0; k < g; ++k) {
@@ -867,8 +872,8 @@ __global__ void __launch_bounds__(warp_cta_warps(G) * 32, 1)
       for (uint32_t k = 0; k < g; ++k) {
         uint4* const st_seed = w_stk + k * p.slots * 32;
         int8_t* const st_t = w_stk_t + k * p.slots * 32;
-        const KeyDev* __restrict__ K = kp + k;
-        const KeyAux* __restrict__ A = ap + k;
+        const KeyDev* K = kp + k;
+        const KeyAux* A = ap + k;
         uint32_t lvl = pi ? M - (uint32_t)__ffs((int)pi) : 0u;
         uint4 s = st_seed[(pi ? lvl - 1 : 0u) * 32];
         uint32_t m = (uint32_t)(int32_t)st_t[(pi ? lvl - 1 : 0u) * 32];
@@ -933,9 +938,9 @@ bool warp_reduces_in_kernel(int G, uint32_t V) { return G > 1 || V > 2; }
 // Block (x, y) = cpb columns x (kThreads / cpb) slices over the partial rows
 // [y * per_block, (y + 1) * per_block); slices combine in shared memory and
 // each block folds its result into out with XOR atomics.
-__global__ void __launch_bounds__(kThreads) reduce_kernel(const uint4* __restrict__ partial,
+__global__ void __launch_bounds__(kThreads) reduce_kernel(const uint4* partial,
                                                           uint32_t nparts, uint32_t cols,
-                                                          uint32_t per_block, uint4* __restrict__ out) {
+                                                          uint32_t per_block, uint4* out) {
   chain_begin();
   __shared__ uint4 red[kThreads];
   const uint32_t cpb = cols < 32u ? cols : 32u;
@@ -958,9 +963,9 @@ __global__ void __launch_bounds__(kThreads) reduce_kernel(const uint4* __restric
 
 // ChaChaKey::eval (dpf.rs:103-142) of one index from its ancestor (s, t) `below`
 // levels above the leaves.
-__device__ __forceinline__ uint4 eval_below(const KeyDev* __restrict__ K, uint4 s, uint32_t t, uint32_t below,
+__device__ __forceinline__ uint4 eval_below(const KeyDev* K, uint4 s, uint32_t t, uint32_t below,
                                             uint64_t x) {
-  const uint32_t d = __ldg(&K->domain_bits);
+  const uint32_t d = K->domain_bits;
 #pragma unroll 1
   for (uint32_t i = below; i-- > 0;) {
     uint4 Lc, Rc;
@@ -984,18 +989,18 @@ __device__ __forceinline__ uint4 eval_below(const KeyDev* __restrict__ K, uint4 
 // with one atomic per word (XOR is order-independent, so the result is
 // deterministic).  The entry count is read on the device so that pushes are
 // seen by replayed graphs.
-__global__ void __launch_bounds__(kThreads) delta_kernel(const KeyDev* __restrict__ keys, const DeltaJob* __restrict__ jobs,
-                                                         const uint4* __restrict__ fr_seed, const uint8_t* __restrict__ fr_t,
-                                                         const uint64_t* __restrict__ idx, const uint4* __restrict__ diffs,
-                                                         const uint32_t* __restrict__ count, uint32_t V, uint64_t first,
-                                                         uint4* __restrict__ out) {
+__global__ void __launch_bounds__(kThreads) delta_kernel(const KeyDev* keys, const DeltaJob* jobs,
+                                                         const uint4* fr_seed, const uint8_t* fr_t,
+                                                         const uint64_t* idx, const uint4* diffs,
+                                                         const uint32_t* count, uint32_t V, uint64_t first,
+                                                         uint4* out) {
   chain_begin();
   __shared__ uint4 s_acc[MG_MAX_ROW_BYTES / 16];
   const uint32_t n = *count;
   const uint64_t e0 = (uint64_t)blockIdx.x * kThreads;
   if (e0 >= n) return;  // uniform per CTA
   const DeltaJob job = jobs[blockIdx.y];
-  const KeyDev* __restrict__ K = keys + job.key;
+  const KeyDev* K = keys + job.key;
   for (uint32_t v = threadIdx.x; v < V; v += kThreads) s_acc[v] = make_uint4(0u, 0u, 0u, 0u);
   const uint64_t e = e0 + threadIdx.x;
   const bool live = e < n;
@@ -1006,7 +1011,7 @@ __global__ void __launch_bounds__(kThreads) delta_kernel(const KeyDev* __restric
       const uint64_t at = job.fr_base + ((x >> job.below) - job.fr_first);
       m = eval_below(K, fr_seed[at], fr_t[at], job.below, x);
     } else {
-      m = eval_below(K, __ldg(&K->root_seed), __ldg(&K->root_t), __ldg(&K->domain_bits), x);
+      m = eval_below(K, K->root_seed, K->root_t, K->domain_bits, x);
     }
   }
   __syncthreads();
@@ -1062,8 +1067,7 @@ __global__ void fill_splitmix_kernel(uint2* __restrict__ dst, uint64_t words, ui
 // at the same time) and the shares out through the pinned host buffers'
 // device-mapped addresses: a kernel node of a few hundred threads finishes
 // sooner than a copy-engine transfer of a few KB.
-__global__ void copy_u4_kernel(const uint4* __restrict__ src, uint4* __restrict__ dst, uint32_t n,
-                               uint4* __restrict__ zero, uint32_t nz) {
+__global__ void copy_u4_kernel(const uint4* src, uint4* dst, uint32_t n, uint4* zero, uint32_t nz) {
   chain_begin();
   const uint32_t m = n > nz ? n : nz;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) {
@@ -1091,7 +1095,7 @@ __global__ void xor_rows_kernel(uint4* __restrict__ table, uint32_t V, const uin
 }
 
 // ChaChaKey::eval (dpf.rs:103-142) at n indices, one thread per index.
-__global__ void eval_points_kernel(const KeyDev* __restrict__ key, const uint64_t* __restrict__ idx,
+__global__ void eval_points_kernel(const KeyDev* key, const uint64_t* __restrict__ idx,
                                    uint64_t n, uint4* __restrict__ out) {
   __shared__ KeyDev sk;
   {
