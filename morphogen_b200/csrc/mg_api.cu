@@ -1102,20 +1102,6 @@ int plan_warp(mg_batch* b, const std::vector<SegPlan>& segs, int G, uint32_t VT,
   const uint64_t nctas = (uint64_t)occ * ctx->sms;
   const uint64_t need_ctas = (items + L.NW - 1) / L.NW;
   L.grid = (uint32_t)std::max<uint64_t>(1, std::min(nctas, need_ctas));
-  // At most one CTA per SM: its shared memory is padded past half an SM's, so
-  // that two never share one.  The CTAs arrive while the frontier still runs
-  // and narrow ones packed onto the SMs it left free (3 keys: 140000 x 128 B
-  // 38.8 us against 47.2, 60000 x 128 B 32.7 against 35.2, 30000 x 128 B 26.3
-  // against 28.2; 12000 x 128 B, two warps a CTA, 24.9 against 28.9; wide CTAs
-  // unchanged).  CTAs of one warp gain nothing from it (4099 x 32 B 25.8 against
-  // 25.2, 2774 x 96 B 23.4 against 22.8) and keep their size.
-  if (L.NW > 1 && L.grid <= (uint32_t)ctx->sms) {
-    const size_t pad = std::min(ctx->smem_optin, ctx->smem_optin / 2 + 2048);
-    if (L.smem < pad) {
-      L.smem = pad;
-      if (int rc = prepare_warp(ctx, G, VT, L.smem)) return rc;
-    }
-  }
   L.nparts = L.grid * L.NW;
   key_cursor = cursor;
   out = std::move(L);

@@ -35,18 +35,31 @@
 
 namespace mg {
 
-// Every kernel of a pass begins with this: it lets the pass's next kernel be
-// launched while this one runs (its CTAs take their places as these leave) and
-// then waits until the kernel before it has completed and its writes are
-// visible.  Nothing in global memory is touched earlier, and what a kernel of
+// Every kernel of a pass begins with one of these two: chain_wait waits until
+// the kernel before it has completed and its writes are visible, chain_begin
+// before that lets the pass's next kernel be launched while this one runs (its
+// CTAs take their places as these leave).
+//
+// The frontier only waits.  A scan launched beside it would hold SMs idle, with
+// most of their shared memory, and any other pass on the device would wait for
+// them; and the CTAs of a narrow scan would crowd onto the SMs that the frontier
+// leaves free.  Launched as the frontier's CTAs end, they spread over the SMs by
+// themselves.  3 keys, two workspaces replaying at once, us per pair of passes
+// with the scan beside its frontier (narrow CTAs padded to one per SM) and
+// after it: 140000 x 128 B 89 and 60, 30000 x 64 B 46 and 28, 175056 x 256 B 100
+// and 70, 2^20 x 256 B 261 and 241; a pass alone: 39.0 and 38.4, 23.0 and 22.8,
+// 43.3 and 43.1, 132.8 and 132.9.
+//
+// Nothing in global memory is touched earlier, and what a kernel of
 // the pass writes (keys, frontier, partial rows, shares) or the host may write
 // beside it (a delta buffer) is read with plain loads: the read-only path and
 // __restrict__ promise data that nothing writes while the kernel lives, and its
 // life now begins before that of its predecessors ends.  Only the table's rows,
 // which no kernel of a pass writes, are read through __ldg.  See launch_chained.
+__device__ __forceinline__ void chain_wait() { cudaGridDependencySynchronize(); }
 __device__ __forceinline__ void chain_begin() {
   cudaTriggerProgrammaticLaunchCompletion();
-  cudaGridDependencySynchronize();
+  chain_wait();
 }
 
 // Up to 4 keys per CTA the kernel is held to 80 registers so that three
@@ -290,7 +303,7 @@ __global__ void __launch_bounds__(kThreads, (G <= 4 ? 3 : 2)) scan_kernel(const 
 // last c - 8 levels are walked depth first, one of the 256 nodes per thread,
 // with no barrier at all.
 __global__ void __launch_bounds__(kThreads) frontier_kernel(const __grid_constant__ FrontierStep f) {
-  chain_begin();
+  chain_wait();
   constexpr uint32_t kWide = 1u << kFrontierWide;  // nodes of the widest breadth-first level
   static_assert(kWide == kThreads, "one node per thread for the depth-first levels");
   __shared__ uint4 sa[kWide], sb[kWide];

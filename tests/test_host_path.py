@@ -123,3 +123,18 @@ def test_graphs_follow_a_delta_buffer_that_keeps_its_index_address(fake, fscanne
     ws.close()
     other.close()
     t.close()
+
+
+@pytest.mark.parametrize("rows,row_bytes", [(12_000, 128), (30_000, 32), (30_000, 64), (60_000, 128), (140_000, 128),
+                                            (100_003, 48), (20_000, 256)])
+def test_narrow_scans_of_two_passes_fit_one_sm(fake, fscanner, rows, row_bytes):
+    # CTAs of a few warps take the shared memory they use and no more, so that
+    # passes of two workspaces can share the SMs.
+    t = G.GpuPageMatrix.alloc_empty(fscanner, rows, row_bytes)
+    ws = fscanner.workspace()
+    ws.set_keys([t] * 3, [key(18, i) for i in range(3)])
+    plan = ws.plan()
+    assert plan["kernel"] == N.KERNEL_WARP and plan["grid"] <= 148
+    assert 2 * (plan["smem_bytes"] + 1024) <= 228 * 1024
+    ws.close()
+    t.close()

@@ -24,10 +24,19 @@ def test_read_only_loads_are_table_rows(path):
 @pytest.mark.parametrize("path", SOURCES, ids=lambda p: p.name)
 def test_chained_kernels_promise_nothing_about_their_arguments(path):
     bodies = re.split(r"__global__", code(path))[1:]
-    chained = [b for b in bodies if "chain_begin();" in b]
+    chained = [b for b in bodies if re.search(r"chain_(begin|wait)\(\);", b)]
     assert bool(chained) == (path.name == "mg_kernels.cu")
     for b in chained:
         assert "__restrict__" not in b[:b.index("{")]
         # Inside, only pointers to the table's rows.
         names = re.findall(r"__restrict__\s+(\w+)", b[b.index("{"):b.index("\n}\n")])
         assert set(names) <= {"tbl", "bp"}
+
+
+def test_a_scan_is_not_launched_beside_its_frontier():
+    # Its idle CTAs would keep other passes off the SMs.
+    bodies = re.split(r"__global__", code(B.CSRC / "mg_kernels.cu"))[1:]
+    (frontier,) = [b for b in bodies if re.match(r"[^{]*\bfrontier_kernel\(", b)]
+    frontier = frontier[:frontier.index("\n}\n")]
+    assert "chain_wait();" in frontier
+    assert "chain_begin" not in frontier and "TriggerProgrammatic" not in frontier
