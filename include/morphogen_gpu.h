@@ -174,7 +174,9 @@ int mg_batch_destroy(mg_batch* batch);
  * workspace stream.  Reallocates device buffers only when they grow. */
 int mg_batch_set_keys(mg_batch* batch, const mg_table* const* tables, const uint8_t* const* keys,
                       const size_t* key_lens, uint32_t nkeys);
-/* Pin the launch shape (0 = let the planner choose). */
+/* Pin the launch shape (0 = let the planner choose).  Rows of up to 512 B that
+ * are no power of two take any shape: 2^6..2^15 rows and 1..4 keys per item on
+ * the warp kernel, the others on the CTA kernel. */
 int mg_batch_set_shape(mg_batch* batch, uint32_t subtree_bits, uint32_t keys_per_cta);
 /* Choose the scan kernel (MG_KERNEL_AUTO by default). */
 int mg_batch_set_kernel(mg_batch* batch, int kind);

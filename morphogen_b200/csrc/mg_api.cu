@@ -797,6 +797,9 @@ int mg_batch_set_kernel(mg_batch* b, int kind) {
 
 namespace {
 
+// Most depth-first levels per lane of the warp kernel.
+constexpr uint32_t kMaxWarpLevels = 10;
+
 // Steps of the frontier chain down to level F, and levels of each but the first.
 constexpr uint32_t kStepLevels = 10;
 uint32_t frontier_steps(uint32_t F) { return F <= kStepLevels ? 1u : (F - 1) / kStepLevels; }
@@ -1009,7 +1012,7 @@ int plan_warp(mg_batch* b, const std::vector<SegPlan>& segs, int G, uint32_t VT,
   };
   std::vector<Cand> cands;
   const uint32_t pinned = b->eff_S;
-  for (uint32_t Mt = 10; Mt >= 1; --Mt) {
+  for (uint32_t Mt = kMaxWarpLevels; Mt >= 1; --Mt) {
     if (pinned && !(pinned >= 6 ? Mt == pinned - 5 : Mt == 1)) continue;
     uint64_t items = 0, nodes = 0;
     double item_nodes = 0, item_loads = 0;
@@ -1197,13 +1200,18 @@ int plan_pass(mg_batch* b) {
 
   // Kernel per segment: the warp kernel for rows of 16..512 B and d >= 1, the
   // CTA kernel otherwise.  A caller may pin the warp kernel for row sizes that
-  // are powers of two only.
+  // are powers of two only; for the others any tile depth and 8 keys per item
+  // may be pinned too, which is the CTA kernel's where the warp kernel has no
+  // such shape (it would refuse the depth or silently take another).
+  const bool warp_shape = (b->eff_S == 0 || (b->eff_S >= 6 && b->eff_S <= kMaxWarpLevels + 5)) &&
+                          (b->eff_G == 0 || mg::warp_g_supported((int)b->eff_G));
   for (SegPlan& sp : segs) {
     const uint32_t V = sp.table->row_bytes / 16;
     const bool ok = mg::warp_vt_supported(V) && sp.d >= 1;
-    if (b->eff_kind == MG_KERNEL_WARP && (!ok || (b->kind_pref == MG_KERNEL_WARP && (V & (V - 1)) != 0)))
+    const bool pow2 = (V & (V - 1)) == 0;
+    if (b->eff_kind == MG_KERNEL_WARP && (!ok || (b->kind_pref == MG_KERNEL_WARP && !pow2)))
       return fail(MG_EINVAL, "the warp kernel needs row_bytes in {16..512, powers of two} and d >= 1");
-    sp.warp = ok && b->eff_kind != MG_KERNEL_CTA;
+    sp.warp = ok && b->eff_kind != MG_KERNEL_CTA && (pow2 || warp_shape);
   }
   // Keys per item: one choice for the CTA kernel, one per row size for the
   // warp kernel (each row size is a launch of its own).

@@ -183,3 +183,22 @@ def test_delta_entries_start_from_the_pass_frontier(scanner, oracle_mod, row_byt
         assert ws.read() == want
     ws.close()
     db.close()
+
+
+@pytest.mark.parametrize("row_bytes", [48, 496])
+@pytest.mark.parametrize("subtree_bits,keys_per_item", [(1, 1), (5, 3), (16, 1), (0, 8), (12, 8)])
+def test_cta_shapes_of_rows_that_are_no_power_of_two(scanner, oracle_mod, row_bytes, subtree_bits, keys_per_item):
+    d, first, nrows, nkeys = 18, 12_345, 9_001, 9
+    db = G.GpuPageMatrix.from_seed(scanner, nrows, row_bytes, seed=6, first_row=first)
+    host = oracle_mod.fill_splitmix(first * row_bytes, nrows * row_bytes, 6).reshape(nrows, row_bytes)
+    keys = [oracle_keypair(oracle_mod, d, first + (7919 * j) % nrows, seed=98, i=j)[0] for j in range(nkeys)]
+    ws = scanner.workspace()
+    ws.set_shape(subtree_bits, keys_per_item)
+    ws.set_keys([db] * nkeys, keys)
+    assert ws.plan()["kernel"] == N.KERNEL_CTA
+    want = oracle_mod.scan_fused(keys, host, row_bytes, row_base=first)
+    for graph in (False, True):
+        ws.launch(graph=graph)
+        assert ws.read() == want
+    ws.close()
+    db.close()

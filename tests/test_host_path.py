@@ -138,3 +138,39 @@ def test_narrow_scans_of_two_passes_fit_one_sm(fake, fscanner, rows, row_bytes):
     assert 2 * (plan["smem_bytes"] + 1024) <= 228 * 1024
     ws.close()
     t.close()
+
+
+@pytest.mark.parametrize("row_bytes", [48, 80, 496])
+@pytest.mark.parametrize("subtree_bits,keys_per_item", [(1, 1), (5, 3), (16, 1), (16, 0), (20, 1), (0, 8), (9, 8)])
+def test_shapes_the_warp_kernel_cannot_take_run_on_the_cta_kernel(fake, fscanner, row_bytes, subtree_bits, keys_per_item):
+    # Items of 2^1..2^5 or more than 2^15 rows, or of eight keys, were valid
+    # for every row size that is no power of two: as CTA tiles.
+    t = G.GpuPageMatrix.alloc_empty(fscanner, 1 << 20, row_bytes)
+    ws = fscanner.workspace()
+    ws.set_shape(subtree_bits, keys_per_item)
+    ws.set_keys([t] * 8, [key(20, i) for i in range(8)])
+    plan = ws.plan()
+    assert plan["kernel"] == N.KERNEL_CTA
+    assert plan["subtree_bits"] == subtree_bits or not subtree_bits
+    assert plan["keys_per_cta"] == keys_per_item or not keys_per_item
+    ws.launch()
+    ws.set_shape(0, 0)
+    ws.set_keys([t] * 8, [key(20, i) for i in range(8)])
+    assert ws.plan()["kernel"] == N.KERNEL_WARP
+    ws.close()
+    t.close()
+
+
+@pytest.mark.parametrize("row_bytes", [48, 80, 496])
+@pytest.mark.parametrize("subtree_bits,keys_per_item", [(6, 1), (15, 1), (9, 3), (0, 4)])
+def test_shapes_the_warp_kernel_takes_stay_on_it(fake, fscanner, row_bytes, subtree_bits, keys_per_item):
+    t = G.GpuPageMatrix.alloc_empty(fscanner, 1 << 20, row_bytes)
+    ws = fscanner.workspace()
+    ws.set_shape(subtree_bits, keys_per_item)
+    ws.set_keys([t] * 4, [key(20, i) for i in range(4)])
+    plan = ws.plan()
+    assert plan["kernel"] == N.KERNEL_WARP
+    assert plan["subtree_bits"] == subtree_bits or not subtree_bits
+    assert plan["keys_per_cta"] == keys_per_item
+    ws.close()
+    t.close()
