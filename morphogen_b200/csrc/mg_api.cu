@@ -185,6 +185,24 @@ struct mg_table {
   uint64_t epoch = 0;
 };
 
+namespace {
+
+// Room in a workspace, in elements of each of its buffers: keys, delta jobs,
+// 16-byte words of partial rows and of shares, frontier nodes and nodes of the
+// frontier chain between its steps.
+struct Room {
+  size_t keys = 0, jobs = 0, partial = 0, out = 0, fr = 0, tmp = 0;
+  bool holds(const Room& r) const {
+    return r.keys <= keys && r.jobs <= jobs && r.partial <= partial && r.out <= out && r.fr <= fr && r.tmp <= tmp;
+  }
+  Room with(const Room& r) const {
+    return {std::max(keys, r.keys), std::max(jobs, r.jobs), std::max(partial, r.partial),
+            std::max(out, r.out),   std::max(fr, r.fr),     std::max(tmp, r.tmp)};
+  }
+};
+
+}  // namespace
+
 struct mg_batch {
   struct Launch {
     int kind = MG_KERNEL_CTA;
@@ -208,20 +226,17 @@ struct mg_batch {
   cudaEvent_t ev_k0 = nullptr, ev_km = nullptr, ev_k1 = nullptr, ev_done = nullptr, ev_h0 = nullptr, ev_h1 = nullptr;
   void* d_arena = nullptr;  // one allocation each for all device and pinned buffers below
   void* h_arena = nullptr;
+  Room cap;                  // what they hold
+  size_t arena_bytes = 0;    // device bytes
   KeyDev* d_keys = nullptr;
   KeyDev* h_keys = nullptr;
-  size_t cap_keys = 0;
   uint4* d_partial = nullptr;
-  size_t cap_partial = 0;
   uint4* d_out = nullptr;
   uint8_t* h_out = nullptr;
-  size_t cap_out = 0;
   uint4* d_fr_seed = nullptr;  // frontier nodes of every warp-kernel key
   uint8_t* d_fr_t = nullptr;
-  size_t cap_fr = 0;
   uint4* d_tmp_seed[2] = {nullptr, nullptr};  // frontier chain intermediates
   uint8_t* d_tmp_t[2] = {nullptr, nullptr};
-  size_t cap_tmp = 0;
   std::vector<Launch> launches;
   struct DeltaLaunch {
     const mg_table* table;
@@ -230,7 +245,6 @@ struct mg_batch {
   std::vector<DeltaLaunch> deltas;
   mg::DeltaJob* d_jobs = nullptr;
   mg::DeltaJob* h_jobs = nullptr;
-  size_t cap_jobs = 0;
   uint32_t total_cols = 0;
   std::vector<uint32_t> key_col;    // first share column of input key i
   std::vector<uint32_t> key_bytes;  // share bytes of input key i
@@ -306,17 +320,38 @@ int prepare_warp(mg_context* ctx, int G, uint32_t VT, size_t smem) {
 // allocation, both pinned ones parts of another, because the first pass of a
 // workspace pays for each call of cudaMalloc (about 0.1 ms; five to nine of
 // them took 0.4 of the 0.7 ms of a first call over 1000003 x 48 B).
-int grow(mg_batch* b, size_t nkeys, size_t njobs, size_t partial_u4, size_t out_u4, size_t fr_nodes,
-         size_t tmp_nodes) {
-  if (nkeys <= b->cap_keys && njobs <= b->cap_jobs && partial_u4 <= b->cap_partial && out_u4 <= b->cap_out &&
-      fr_nodes <= b->cap_fr && tmp_nodes <= b->cap_tmp)
-    return MG_OK;
-  nkeys = std::max(nkeys, b->cap_keys);
-  njobs = std::max(njobs, b->cap_jobs);
-  partial_u4 = std::max(partial_u4, b->cap_partial);
-  out_u4 = std::max(out_u4, b->cap_out);
-  fr_nodes = std::max(fr_nodes, b->cap_fr);
-  tmp_nodes = std::max(tmp_nodes, b->cap_tmp);
+//
+// Where the parts of `room` lie in the two allocations.
+struct Layout {
+  size_t keys, out, jobs, host_bytes, partial, fr, fr_t, tmp[2], tmp_t[2], bytes;
+};
+Layout layout_of(const Room& room) {
+  Layout l;
+  size_t bytes = 0;
+  auto part = [&](size_t n) {
+    const size_t at = bytes;
+    bytes += (n + 255) / 256 * 256;
+    return at;
+  };
+  // Keys, then their warp-kernel constants (KeyAux) right after the pass's keys.
+  l.keys = part(room.keys * (sizeof(KeyDev) + sizeof(mg::KeyAux)));
+  l.out = part(room.out * 16);
+  l.jobs = part(room.jobs * sizeof(mg::DeltaJob));
+  l.host_bytes = bytes;
+  l.partial = part(room.partial * 16);
+  l.fr = part(room.fr * 16);
+  l.fr_t = part(room.fr);
+  for (int i = 0; i < 2; ++i) {
+    l.tmp[i] = part(room.tmp * 16);
+    l.tmp_t[i] = part(room.tmp);
+  }
+  l.bytes = bytes;
+  return l;
+}
+
+int grow(mg_batch* b, const Room& need) {
+  if (b->cap.holds(need)) return MG_OK;
+  Room room = b->cap.with(need);
   b->planned = false;  // the old plan's pointers go with the old allocation
   b->d_keys = b->h_keys = nullptr;
   b->d_jobs = b->h_jobs = nullptr;
@@ -326,52 +361,39 @@ int grow(mg_batch* b, size_t nkeys, size_t njobs, size_t partial_u4, size_t out_
   if (b->h_arena) cudaFreeHost(b->h_arena);
   b->d_arena = nullptr;
   b->h_arena = nullptr;
-  b->cap_keys = b->cap_jobs = b->cap_partial = b->cap_out = b->cap_fr = b->cap_tmp = 0;
-  size_t bytes = 0;
-  auto part = [&](size_t n) {
-    const size_t at = bytes;
-    bytes += (n + 255) / 256 * 256;
-    return at;
-  };
-  // Keys, then their warp-kernel constants (KeyAux) right after the pass's keys.
-  const size_t key_bytes = nkeys * (sizeof(KeyDev) + sizeof(mg::KeyAux));
-  const size_t keys_at = part(key_bytes), out_at = part(out_u4 * 16), jobs_at = part(njobs * sizeof(mg::DeltaJob));
-  const size_t host_bytes = bytes;
-  const size_t partial_at = part(partial_u4 * 16), fr_at = part(fr_nodes * 16), fr_t_at = part(fr_nodes);
-  size_t tmp_at[2], tmp_t_at[2];
-  for (int i = 0; i < 2; ++i) {
-    tmp_at[i] = part(tmp_nodes * 16);
-    tmp_t_at[i] = part(tmp_nodes);
-  }
-  if (cudaMalloc(&b->d_arena, bytes) != cudaSuccess || cudaMallocHost(&b->h_arena, host_bytes) != cudaSuccess) {
+  b->cap = Room();
+  b->arena_bytes = 0;
+  // With what earlier passes needed, or else without.
+  Layout at = layout_of(room);
+  while (cudaMalloc(&b->d_arena, at.bytes) != cudaSuccess ||
+         cudaMallocHost(&b->h_arena, at.host_bytes) != cudaSuccess) {
     cudaGetLastError();
     if (b->d_arena) cudaFree(b->d_arena);
     b->d_arena = nullptr;
     b->h_arena = nullptr;
-    b->launched = false;  // the last pass's shares are gone too
-    return fail(MG_ENOMEM, "cannot allocate %zu bytes of workspace for %zu keys", bytes, nkeys);
+    if (need.holds(room)) {
+      b->launched = false;  // the last pass's shares are gone too
+      return fail(MG_ENOMEM, "cannot allocate %zu bytes of workspace for %zu keys", at.bytes, need.keys);
+    }
+    at = layout_of(room = need);
   }
-  auto dev = [&](size_t at) { return static_cast<uint8_t*>(b->d_arena) + at; };
-  auto host = [&](size_t at) { return static_cast<uint8_t*>(b->h_arena) + at; };
-  b->d_keys = reinterpret_cast<KeyDev*>(dev(keys_at));
-  b->h_keys = reinterpret_cast<KeyDev*>(host(keys_at));
-  b->d_out = reinterpret_cast<uint4*>(dev(out_at));
-  b->h_out = host(out_at);
-  b->d_jobs = reinterpret_cast<mg::DeltaJob*>(dev(jobs_at));
-  b->h_jobs = reinterpret_cast<mg::DeltaJob*>(host(jobs_at));
-  b->d_partial = reinterpret_cast<uint4*>(dev(partial_at));
-  b->d_fr_seed = reinterpret_cast<uint4*>(dev(fr_at));
-  b->d_fr_t = dev(fr_t_at);
+  auto dev = [&](size_t o) { return static_cast<uint8_t*>(b->d_arena) + o; };
+  auto host = [&](size_t o) { return static_cast<uint8_t*>(b->h_arena) + o; };
+  b->d_keys = reinterpret_cast<KeyDev*>(dev(at.keys));
+  b->h_keys = reinterpret_cast<KeyDev*>(host(at.keys));
+  b->d_out = reinterpret_cast<uint4*>(dev(at.out));
+  b->h_out = host(at.out);
+  b->d_jobs = reinterpret_cast<mg::DeltaJob*>(dev(at.jobs));
+  b->h_jobs = reinterpret_cast<mg::DeltaJob*>(host(at.jobs));
+  b->d_partial = reinterpret_cast<uint4*>(dev(at.partial));
+  b->d_fr_seed = reinterpret_cast<uint4*>(dev(at.fr));
+  b->d_fr_t = dev(at.fr_t);
   for (int i = 0; i < 2; ++i) {
-    b->d_tmp_seed[i] = reinterpret_cast<uint4*>(dev(tmp_at[i]));
-    b->d_tmp_t[i] = dev(tmp_t_at[i]);
+    b->d_tmp_seed[i] = reinterpret_cast<uint4*>(dev(at.tmp[i]));
+    b->d_tmp_t[i] = dev(at.tmp_t[i]);
   }
-  b->cap_keys = nkeys;
-  b->cap_jobs = njobs;
-  b->cap_partial = partial_u4;
-  b->cap_out = out_u4;
-  b->cap_fr = fr_nodes;
-  b->cap_tmp = tmp_nodes;
+  b->cap = room;
+  b->arena_bytes = at.bytes;
   return MG_OK;
 }
 
@@ -884,7 +906,7 @@ size_t wire_frontier(mg_batch* b, mg_batch::Launch& L, size_t st, uint32_t F, ui
 // 30000 x 4 KB: 54 at 7, 67 at 6, 61 at 8).
 int plan_cta(mg_batch* b, const std::vector<SegPlan>& segs, int G, uint32_t col0, size_t& key_cursor,
              std::vector<uint32_t>& key_col, std::vector<uint32_t>& key_bytes, std::vector<uint32_t>& key_slot,
-             uint64_t& fr_cursor, size_t& tmp_need, mg_batch::Launch& out) {
+             uint64_t& fr_cursor, size_t& tmp_need, bool frontier, mg_batch::Launch& out) {
   mg_context* ctx = b->ctx;
   for (uint32_t S_target = b->eff_S ? b->eff_S : 14;; --S_target) {
     mg_batch::Launch L;
@@ -953,7 +975,7 @@ int plan_cta(mg_batch* b, const std::vector<SegPlan>& segs, int G, uint32_t col0
       // with one item each, the walk inside the kernel is shorter than another
       // launch (3 keys, 3000 x 4 KB: 57 us against 64; 200000 x 4 KB, 1.8 items
       // per CTA: 191 against 186; 500000 x 1 KB: 189 against 166).
-      if (items > L.grid) {
+      if (frontier && items > L.grid) {
         fr_cursor = fr;
         tmp_need = tmp;
       } else {
@@ -993,11 +1015,12 @@ double warp_cost_us(uint64_t items, double item_nodes, double item_loads, uint64
 }
 
 // Plan one warp-kernel launch over segs (same V, at most kMaxSegs): depth-first
-// levels per lane M (the cheapest by warp_cost_us, or pinned as subtree_bits =
-// M + 5) and the CTA width.
+// levels per lane M (the cheapest of min_levels and more by warp_cost_us, or
+// pinned as subtree_bits = M + 5) and the CTA width.
 int plan_warp(mg_batch* b, const std::vector<SegPlan>& segs, int G, uint32_t VT, uint32_t col0,
               size_t& key_cursor, std::vector<uint32_t>& key_col, std::vector<uint32_t>& key_bytes,
-              std::vector<uint32_t>& key_slot, uint64_t& fr_cursor, size_t& tmp_need, mg_batch::Launch& out) {
+              std::vector<uint32_t>& key_slot, uint64_t& fr_cursor, size_t& tmp_need, uint32_t min_levels,
+              mg_batch::Launch& out) {
   mg_context* ctx = b->ctx;
   struct Shape { uint32_t slots, nw; size_t smem; };
   struct Cand { uint32_t M; double cost; Shape sh; };
@@ -1012,7 +1035,7 @@ int plan_warp(mg_batch* b, const std::vector<SegPlan>& segs, int G, uint32_t VT,
   };
   std::vector<Cand> cands;
   const uint32_t pinned = b->eff_S;
-  for (uint32_t Mt = kMaxWarpLevels; Mt >= 1; --Mt) {
+  for (uint32_t Mt = kMaxWarpLevels; Mt >= (pinned ? 1u : min_levels); --Mt) {
     if (pinned && !(pinned >= 6 ? Mt == pinned - 5 : Mt == 1)) continue;
     uint64_t items = 0, nodes = 0;
     double item_nodes = 0, item_loads = 0;
@@ -1179,6 +1202,97 @@ mg::DeltaJob delta_job(const std::vector<mg_batch::Launch>& launches, const mg_t
   return job;
 }
 
+// What a pass launches, and the room it needs.
+struct Plan {
+  std::vector<mg_batch::Launch> launches;
+  std::vector<mg_batch::DeltaLaunch> deltas;
+  std::vector<mg::DeltaJob> jobs;
+  std::vector<uint32_t> key_col, key_bytes, key_slot;
+  Room need;
+};
+
+// Launches: CTA-kernel segments in chunks of kMaxSegs; warp-kernel segments
+// grouped by V, then chunks of kMaxSegs.  min_levels: see plan_pass.
+int plan_launches(mg_batch* b, const std::vector<SegPlan>& split, int Gc, const std::map<uint32_t, int>& Gw,
+                  uint32_t min_levels, Plan& P) {
+  const uint32_t nkeys = (uint32_t)b->in_keys.size();
+  P = Plan();
+  std::vector<mg_batch::Launch>& launches = P.launches;
+  std::vector<uint32_t>&key_col = P.key_col, &key_bytes = P.key_bytes, &key_slot = P.key_slot;
+  key_col.resize(nkeys);
+  key_bytes.resize(nkeys);
+  key_slot.resize(nkeys);
+  size_t key_cursor = 0, tmp_need = 0;
+  uint64_t fr_cursor = 0;
+  uint32_t total_cols = 0;
+  std::vector<SegPlan> cta_segs;
+  for (const SegPlan& sp : split)
+    if (!sp.warp) cta_segs.push_back(sp);
+  for (size_t s0 = 0; s0 < cta_segs.size(); s0 += mg::kMaxSegs) {
+    std::vector<SegPlan> chunk(cta_segs.begin() + s0,
+                               cta_segs.begin() + std::min(cta_segs.size(), s0 + mg::kMaxSegs));
+    mg_batch::Launch L;
+    if (int rc = plan_cta(b, chunk, Gc, total_cols, key_cursor, key_col, key_bytes, key_slot, fr_cursor, tmp_need,
+                          min_levels == 1, L))
+      return rc;
+    total_cols += L.cols;
+    launches.push_back(std::move(L));
+  }
+  for (const auto& vg : Gw) {
+    const uint32_t VT = vg.first;
+    std::vector<SegPlan> ws;
+    for (const SegPlan& sp : split)
+      if (sp.warp && sp.table->row_bytes / 16 == VT) ws.push_back(sp);
+    for (size_t s0 = 0; s0 < ws.size(); s0 += mg::kMaxSegs) {
+      std::vector<SegPlan> chunk(ws.begin() + s0, ws.begin() + std::min(ws.size(), s0 + mg::kMaxSegs));
+      mg_batch::Launch L;
+      if (int rc = plan_warp(b, chunk, vg.second, VT, total_cols, key_cursor, key_col, key_bytes, key_slot, fr_cursor,
+                             tmp_need, min_levels, L))
+        return rc;
+      total_cols += L.cols;
+      launches.push_back(std::move(L));
+    }
+  }
+
+  // Delta folding: one launch per table that holds a delta buffer.
+  std::vector<mg_batch::DeltaLaunch>& deltas = P.deltas;
+  std::vector<mg::DeltaJob>& jobs = P.jobs;
+  for (uint32_t i = 0; i < nkeys; ++i) {
+    const mg_table* t = b->in_tables[i];
+    if (!t->delta_cap) continue;
+    auto it = std::find_if(deltas.begin(), deltas.end(), [&](const mg_batch::DeltaLaunch& x) { return x.table == t; });
+    if (it == deltas.end()) {
+      deltas.push_back({t, 0, 0});
+      it = deltas.end() - 1;
+    }
+  }
+  for (mg_batch::DeltaLaunch& dl : deltas) {
+    dl.job0 = (uint32_t)jobs.size();
+    for (uint32_t i = 0; i < nkeys; ++i)
+      if (b->in_tables[i] == dl.table) jobs.push_back(delta_job(launches, dl.table, key_slot[i], key_col[i]));
+    dl.njobs = (uint32_t)jobs.size() - dl.job0;
+  }
+
+  size_t max_partial = 0;
+  for (const mg_batch::Launch& L : launches) max_partial = std::max(max_partial, (size_t)L.nparts * L.cols);
+  P.need = {nkeys, jobs.size(), max_partial, total_cols, (size_t)fr_cursor, tmp_need};
+  return MG_OK;
+}
+
+// Whether the room a plan needs, if the workspace has to grow for it, is more
+// than a quarter of the free memory (asked for above 256 MiB only).
+bool scratch_too_large(const mg_batch* b, const Room& need) {
+  if (b->cap.holds(need)) return false;
+  const size_t bytes = layout_of(need).bytes;
+  if (bytes <= (size_t)256 << 20) return false;
+  size_t free_b = 0, total_b = 0;
+  if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return bytes > (free_b + b->arena_bytes) / 4;
+}
+
 // Plan the pass for b->in_keys / b->in_tables with the effective shape
 // (b->eff_kind, b->eff_S, b->eff_G), allocate, stage the keys and copy them
 // to the device on the workspace stream.
@@ -1241,67 +1355,31 @@ int plan_pass(mg_batch* b) {
                               (uint32_t)(sp.keys.size() - full), sp.warp});
   }
 
-  // Launches: CTA-kernel segments in chunks of kMaxSegs; warp-kernel segments
-  // grouped by V, then chunks of kMaxSegs.
-  std::vector<mg_batch::Launch> launches;
-  std::vector<uint32_t> key_col(nkeys), key_bytes(nkeys), key_slot(nkeys);
-  size_t key_cursor = 0, tmp_need = 0;
-  uint64_t fr_cursor = 0;
-  uint32_t total_cols = 0;
-  std::vector<SegPlan> cta_segs;
-  for (const SegPlan& sp : split)
-    if (!sp.warp) cta_segs.push_back(sp);
-  for (size_t s0 = 0; s0 < cta_segs.size(); s0 += mg::kMaxSegs) {
-    std::vector<SegPlan> chunk(cta_segs.begin() + s0,
-                               cta_segs.begin() + std::min(cta_segs.size(), s0 + mg::kMaxSegs));
-    mg_batch::Launch L;
-    if (int rc = plan_cta(b, chunk, Gc, total_cols, key_cursor, key_col, key_bytes, key_slot, fr_cursor, tmp_need, L)) return rc;
-    total_cols += L.cols;
-    launches.push_back(std::move(L));
+  // The fastest plan, or, where its frontier does not fit the memory or would
+  // take more than a quarter of what is free, the fastest one with at least two,
+  // three, ... depth-first levels per lane (and no frontier for the CTA kernel):
+  // with 10 levels it is a node for 1024 rows and key, where the fastest plan of
+  // a wide-row table has up to one for 8 (17 GB for 48 keys over 340000000 x
+  // 512 B).
+  Plan P;
+  for (uint32_t min_levels = 1;; ++min_levels) {
+    if (int rc = plan_launches(b, split, Gc, Gw, min_levels, P)) return rc;
+    const bool last = min_levels == kMaxWarpLevels;
+    if (!last && scratch_too_large(b, P.need)) continue;
+    const int rc = grow(b, P.need);
+    if (rc == MG_OK) break;
+    if (last || rc != MG_ENOMEM) return rc;
   }
-  for (const auto& vg : Gw) {
-    const uint32_t VT = vg.first;
-    std::vector<SegPlan> ws;
-    for (const SegPlan& sp : split)
-      if (sp.warp && sp.table->row_bytes / 16 == VT) ws.push_back(sp);
-    for (size_t s0 = 0; s0 < ws.size(); s0 += mg::kMaxSegs) {
-      std::vector<SegPlan> chunk(ws.begin() + s0, ws.begin() + std::min(ws.size(), s0 + mg::kMaxSegs));
-      mg_batch::Launch L;
-      if (int rc = plan_warp(b, chunk, vg.second, VT, total_cols, key_cursor, key_col, key_bytes, key_slot, fr_cursor,
-                             tmp_need, L))
-        return rc;
-      total_cols += L.cols;
-      launches.push_back(std::move(L));
-    }
-  }
-
-  // Delta folding: one launch per table that holds a delta buffer.
-  std::vector<mg_batch::DeltaLaunch> deltas;
-  std::vector<mg::DeltaJob> jobs;
-  for (uint32_t i = 0; i < nkeys; ++i) {
-    const mg_table* t = b->in_tables[i];
-    if (!t->delta_cap) continue;
-    auto it = std::find_if(deltas.begin(), deltas.end(), [&](const mg_batch::DeltaLaunch& x) { return x.table == t; });
-    if (it == deltas.end()) {
-      deltas.push_back({t, 0, 0});
-      it = deltas.end() - 1;
-    }
-  }
-  for (mg_batch::DeltaLaunch& dl : deltas) {
-    dl.job0 = (uint32_t)jobs.size();
-    for (uint32_t i = 0; i < nkeys; ++i)
-      if (b->in_tables[i] == dl.table) jobs.push_back(delta_job(launches, dl.table, key_slot[i], key_col[i]));
-    dl.njobs = (uint32_t)jobs.size() - dl.job0;
-  }
-
-  size_t max_partial = 0;
-  for (const mg_batch::Launch& L : launches) max_partial = std::max(max_partial, (size_t)L.nparts * L.cols);
-  if (int rc = grow(b, nkeys, jobs.size(), max_partial, total_cols, (size_t)fr_cursor, tmp_need)) return rc;
+  std::vector<mg_batch::Launch>& launches = P.launches;
+  std::vector<uint32_t>&key_col = P.key_col, &key_bytes = P.key_bytes, &key_slot = P.key_slot;
+  std::vector<mg::DeltaJob>& jobs = P.jobs;
+  const uint32_t total_cols = (uint32_t)P.need.out;
+  const uint64_t fr_cursor = P.need.fr;
   if (!jobs.empty()) {
     std::memcpy(b->h_jobs, jobs.data(), jobs.size() * sizeof(mg::DeltaJob));
     MG_CUDA(cudaMemcpyAsync(b->d_jobs, b->h_jobs, jobs.size() * sizeof(mg::DeltaJob), cudaMemcpyHostToDevice, b->stream));
   }
-  b->deltas = std::move(deltas);
+  b->deltas = std::move(P.deltas);
   mg::KeyAux* const h_aux = reinterpret_cast<mg::KeyAux*>(b->h_keys + nkeys);
   const mg::KeyAux* const d_aux = reinterpret_cast<const mg::KeyAux*>(b->d_keys + nkeys);
   for (uint32_t i = 0; i < nkeys; ++i) {
