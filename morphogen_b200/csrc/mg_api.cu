@@ -228,6 +228,7 @@ struct mg_batch {
   void* h_arena = nullptr;
   Room cap;                  // what they hold
   size_t arena_bytes = 0;    // device bytes
+  size_t scratch_limit = 0;  // device bytes they are to stay within (0: see scratch_too_large)
   KeyDev* d_keys = nullptr;
   KeyDev* h_keys = nullptr;
   uint4* d_partial = nullptr;
@@ -365,6 +366,7 @@ int grow(mg_batch* b, const Room& need) {
   b->arena_bytes = 0;
   // With what earlier passes needed, or else without.
   Layout at = layout_of(room);
+  if (b->scratch_limit && at.bytes > b->scratch_limit) at = layout_of(room = need);
   while (cudaMalloc(&b->d_arena, at.bytes) != cudaSuccess ||
          cudaMallocHost(&b->h_arena, at.host_bytes) != cudaSuccess) {
     cudaGetLastError();
@@ -1280,10 +1282,12 @@ int plan_launches(mg_batch* b, const std::vector<SegPlan>& split, int Gc, const 
 }
 
 // Whether the room a plan needs, if the workspace has to grow for it, is more
-// than a quarter of the free memory (asked for above 256 MiB only).
+// than the limit set for it or, without one, than a quarter of the free memory
+// (asked for above 256 MiB only).
 bool scratch_too_large(const mg_batch* b, const Room& need) {
   if (b->cap.holds(need)) return false;
   const size_t bytes = layout_of(need).bytes;
+  if (b->scratch_limit) return bytes > b->scratch_limit;
   if (bytes <= (size_t)256 << 20) return false;
   size_t free_b = 0, total_b = 0;
   if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
@@ -1356,7 +1360,8 @@ int plan_pass(mg_batch* b) {
   }
 
   // The fastest plan, or, where its frontier does not fit the memory or would
-  // take more than a quarter of what is free, the fastest one with at least two,
+  // take more than a quarter of what is free (or than a server may let it have),
+  // the fastest one with at least two,
   // three, ... depth-first levels per lane (and no frontier for the CTA kernel):
   // with 10 levels it is a node for 1024 rows and key, where the fastest plan of
   // a wide-row table has up to one for 8 (17 GB for 48 keys over 340000000 x
@@ -2030,5 +2035,6 @@ bool batch_done(mg_batch* b) {
   cudaGetLastError();
   return true;
 }
+void batch_limit_growth(mg_batch* b, uint64_t bytes) { b->scratch_limit = (size_t)bytes + b->arena_bytes + 1; }
 int context_device(const mg_context* ctx) { return ctx->device; }
 }  // namespace mg

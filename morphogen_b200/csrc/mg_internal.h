@@ -59,6 +59,9 @@ namespace mg {
 
 // True once the workspace's last enqueued work has completed on the device.
 bool batch_done(mg_batch* b);
+// Plans made from now on let the workspace grow by at most `bytes` of device
+// memory where a plan with a smaller frontier does.
+void batch_limit_growth(mg_batch* b, uint64_t bytes);
 int context_device(const mg_context* ctx);
 
 // Sets the thread-local message returned by mg_last_error().

@@ -55,20 +55,15 @@ struct Request {
   bool done = false;
 };
 
-// Device bytes a key adds to a pass: its device copy (key and warp-kernel
-// constants, 1264 B), its frontier (17 B per node: at most rows / 2 nodes for
-// tables up to 2^24 rows; above, a lone key's planned depth grows by one level
-// per factor of four in rows, from 6 levels at 2^25 to 9 at 2^31, and is
-// deeper with more keys) and partial-row columns for every persistent warp.
+// Device bytes a key needs in a pass: its device copy (key and warp-kernel
+// constants), its frontier (17 B per node) and partial-row columns for every
+// persistent warp.  The frontier counted is at most a node for 2 rows, for 256
+// of tables above 2^24 rows: the planner takes a larger one where that is
+// faster, but not beyond the growth a pass is allowed (batch_limit_growth), and
+// it can go down to a node for 1024 rows.
 uint64_t key_scratch_bytes(const mg_table* t, int sms) {
   const uint64_t rows = mg_table_rows(t);
-  uint32_t shift = 1;
-  if (rows > (1ull << 24)) {
-    uint32_t lg = 24;
-    while (lg < 32 && (1ull << lg) < rows) ++lg;
-    shift = (lg - 14) / 2;
-  }
-  const uint64_t frontier = (rows >> shift) * 17 + 32 * 17;
+  const uint64_t frontier = (rows <= (1ull << 24) ? rows / 2 : rows >> 8) * 17 + 32 * 17;
   const uint64_t partial = (uint64_t)sms * 4 * 8 * (mg_table_row_bytes(t));
   return sizeof(mg::KeyDev) + sizeof(mg::KeyAux) + frontier + partial;
 }
@@ -211,6 +206,9 @@ void run(mg_server* s) {
         s->slot_reqs[i] = take;
         s->slot_cost[i] = cost;
         lk.unlock();
+        // What the pass was admitted with, or more where all slots together
+        // still leave half of the budget.
+        mg::batch_limit_growth(s->slots[i], std::max(need, budget / (2 * s->slots.size())));
         int rc = mg_batch_set_keys(s->slots[i], tabs.data(), kp.data(), kl.data(), (uint32_t)kp.size());
         if (rc == MG_OK) rc = mg_batch_launch(s->slots[i], nullptr);
         std::string err = rc == MG_OK ? std::string() : std::string(mg_last_error());

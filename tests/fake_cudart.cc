@@ -41,7 +41,7 @@ struct Launch {
 };
 
 std::mutex mu;
-uint64_t capacity = 178ull << 30, used = 0, next_addr = kBase;
+uint64_t capacity = 178ull << 30, used = 0, peak = 0, next_addr = kBase;
 bool reuse = false;                                  // freed addresses are handed out again (exact size)
 std::map<uint64_t, uint64_t> live;                   // address -> bytes
 std::map<uint64_t, std::vector<uint64_t>> freed;     // bytes -> addresses
@@ -131,9 +131,11 @@ void fake_reset(uint64_t bytes, int reuse_addresses) {
   capacity = bytes;
   reuse = reuse_addresses != 0;
   fail_mask = dead_launches = graphs = 0;
+  peak = used;
 }
 void fake_fail(uint64_t mask) { fail_mask = mask; }
 uint64_t fake_used() { return used; }
+uint64_t fake_peak() { return peak; }
 uint64_t fake_dead_launches() { return dead_launches; }
 uint64_t fake_graphs() { return graphs; }
 void fake_last_delta(uint64_t out[4]) { std::memcpy(out, last_delta, sizeof last_delta); }
@@ -204,6 +206,7 @@ cudaError_t cudaMalloc(void** p, size_t n) {
   }
   live[a] = n;
   used += n;
+  peak = std::max(peak, used);
   *p = (void*)a;
   return cudaSuccess;
 }

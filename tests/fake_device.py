@@ -51,7 +51,7 @@ def fake_library(path: Path):
         L.fake_reset.argtypes = [C.c_uint64, C.c_int]
         L.fake_fail.argtypes = [C.c_uint64]
         L.fake_last_delta.argtypes = [C.c_uint64 * 4]
-        for f in (L.fake_used, L.fake_dead_launches, L.fake_graphs):
+        for f in (L.fake_used, L.fake_peak, L.fake_dead_launches, L.fake_graphs):
             f.restype = C.c_uint64
         gc.enable()
         yield L

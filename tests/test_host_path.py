@@ -8,6 +8,7 @@ import pytest
 import fake_device
 from morphogen_b200 import _native as N
 from morphogen_b200 import gpu_dpf as G
+from morphogen_b200.server import PirServer
 
 
 @pytest.fixture(scope="module")
@@ -241,4 +242,24 @@ def test_pinned_cta_tiles_need_no_frontier_when_it_does_not_fit(fake, fscanner, 
     ws.launch()
     assert fake.fake_dead_launches() == 0
     ws.close()
+    t.close()
+
+
+@pytest.mark.parametrize("rows,row_bytes,nkeys", BIG)
+@pytest.mark.parametrize("slots", [1, 2])
+def test_a_server_keeps_its_memory_reserve(fake, fscanner, rows, row_bytes, nkeys, slots):
+    # Budget for a third of the requests at once: passes take as many as are
+    # admitted, none fails and the reserve is never touched.
+    d, lookups = (rows - 1).bit_length(), max(3, nkeys)
+    reserve, budget = 1 << 30, slots * (scratch(rows, row_bytes, (lookups + 2) // 3) + (1 << 20))
+    fake.fake_reset(rows * row_bytes + budget + reserve, 0)
+    t = G.GpuPageMatrix.alloc_empty(fscanner, rows, row_bytes)
+    srv = PirServer(fscanner, slots=slots, max_keys_per_pass=lookups, memory_reserve=reserve)
+    ids = [srv.submit([(t, key(d, i))]) for i in range(lookups)]
+    for i in ids:
+        assert len(srv.wait(i, 20_000)[0]) == 1
+    stats = srv.stats()
+    srv.close()
+    assert stats["completed"] == lookups and stats["failed"] == 0
+    assert fake.fake_peak() <= rows * row_bytes + budget
     t.close()
