@@ -20,6 +20,7 @@
 #include <algorithm>
 #include <chrono>
 #include <condition_variable>
+#include <cstdint>
 #include <cstring>
 #include <deque>
 #include <mutex>
@@ -158,6 +159,7 @@ void run(mg_server* s) {
     if (s->stop && in_flight(s) == 0) break;
     // 2. Dispatch: one pass per free workspace from everything pending.
     if (!s->paused && !s->stop) {
+      size_t max_take = SIZE_MAX;  // requests of the next pass
       for (size_t i = 0; i < s->slots.size() && !s->pending.empty(); ++i) {
         if (!s->slot_reqs[i].empty()) continue;
         size_t free_b = 0, total_b = 0;
@@ -177,7 +179,7 @@ void run(mg_server* s) {
         std::vector<Request*> take;
         uint64_t need = 0, nk = 0;
         double cost = 0;
-        while (!s->pending.empty()) {
+        while (!s->pending.empty() && take.size() < max_take) {
           Request* r = s->pending.front();
           const bool first = take.empty();
           if (!first && s->cfg.max_keys_per_pass && nk + r->keys.size() > s->cfg.max_keys_per_pass) break;
@@ -214,17 +216,24 @@ void run(mg_server* s) {
         std::string err = rc == MG_OK ? std::string() : std::string(mg_last_error());
         lk.lock();
         if (rc != MG_OK) {
-          if (rc == MG_ENOMEM && in_flight(s) > 1) {
-            // Memory is held by other passes: put the requests back in order.
+          if (rc == MG_ENOMEM && (in_flight(s) > 1 || take.size() > 1)) {
+            // Put the requests back in order.  Memory is held by other passes,
+            // which are waited for, or there is none for a pass of so many:
+            // half of them are tried.
             for (auto it = take.rbegin(); it != take.rend(); ++it) s->pending.push_front(*it);
             s->slot_reqs[i].clear();
-            break;
+            s->cv_done.notify_all();  // a pause may be waiting for this slot
+            if (in_flight(s) > 0) break;
+            max_take = take.size() / 2;
+            --i;
+            continue;
           }
           finish_slot(s, i, rc, err.c_str(), {});
           s->cv_done.notify_all();
           continue;
         }
         s->slot_start[i] = Clock::now();
+        max_take = SIZE_MAX;
       }
     }
     // 3. Sleep until new work or (briefly) to poll the GPU.

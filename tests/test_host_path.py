@@ -263,3 +263,28 @@ def test_a_server_keeps_its_memory_reserve(fake, fscanner, rows, row_bytes, nkey
     assert stats["completed"] == lookups and stats["failed"] == 0
     assert fake.fake_peak() <= rows * row_bytes + budget
     t.close()
+
+
+@pytest.mark.parametrize("slots", [1, 2])
+def test_a_server_splits_a_pass_that_finds_no_memory(fake, fscanner, slots):
+    # Device memory that others take between the admission and the pass: all
+    # of the pass's tries fail (and, later, those of its half).
+    t = G.GpuPageMatrix.alloc_empty(fscanner, 5000, 32)
+    srv = PirServer(fscanner, slots=slots, max_keys_per_pass=12)
+    srv.pause()
+    ids = [srv.submit([(t, key(13, i))]) for i in range(24)]
+    fake.fake_fail((1 << 20) - 1)
+    srv.resume()
+    for i in ids:
+        assert len(srv.wait(i, 20_000)[0]) == 1
+    stats = srv.stats()
+    assert stats["completed"] == 24 and stats["failed"] == 0 and stats["passes"] >= 3
+    srv.close()
+    # One request alone that finds none is answered with the error.
+    srv = PirServer(fscanner, slots=slots)
+    fake.fake_reset(fake.fake_used(), 0)
+    with pytest.raises(N.MgError) as err:
+        srv.wait(srv.submit([(t, key(13, 0))]), 20_000)
+    assert err.value.code == N.MG_ENOMEM
+    srv.close()
+    t.close()
