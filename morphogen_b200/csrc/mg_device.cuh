@@ -13,7 +13,7 @@
 // (456 instructions) and the FMA pipe half idle (227).  Rotations by 16 and 8
 // are whole bytes, and a byte-wise dot product plus a multiply-add does one on
 // the FMA pipe (rotl_bytes): with 70 of them there, about 387 ALU and 366 FMA
-// instructions, 40.2 -> 44.6 G node expansions/s for the PRG alone
+// instructions, 40.2 -> 45.2 G node expansions/s for the PRG alone
 // (mg_prg_peak).  More of them loses to the issue rate (one instruction per
 // clock and scheduler, 755 per expansion), fewer to the ALU pipe.  Both blocks
 // are written out in one straight-line function so the compiler shares the
@@ -344,7 +344,7 @@ struct WarpSeg {
   uint64_t fr_base;     // frontier index of the segment's key 0 (key j at fr_base + j * nF)
   uint64_t nF;          // frontier nodes per key (level d - M nodes meeting the rows)
   uint32_t tiles;       // warp tiles per key group = ceil(nF / 32)
-  uint32_t groups;      // key groups (items are group-major)
+  uint32_t groups;      // key groups (items are tile-major: the groups of a tile lie side by side)
   uint32_t d;           // domain bits
   uint32_t M;           // depth-first levels per lane (>= 1)
   uint32_t g;           // keys per group

@@ -11,10 +11,10 @@ namespace mg {
 
 size_t scan_smem_bytes(int G, uint32_t slots);
 bool scan_g_supported(int G);
+bool scan_fma(uint32_t V);  // which of the kernel's two PRG forms rows of V uint4 take
 // Raise (never lower) the kernel's dynamic shared memory limit on the current
 // device to at least smem.  The limit is process-wide per device and kernel,
 // so every caller goes through this one record (scan_prepare / warp_prepare).
-bool scan_fma(uint32_t V);  // which of the kernel's two PRG forms rows of V uint4 take
 cudaError_t scan_prepare(int G, bool fma, size_t smem);
 int scan_occupancy(int G, bool fma, size_t smem);
 cudaError_t launch_scan(int G, bool fma, const ScanParams& p, uint32_t grid, size_t smem, cudaStream_t st);
@@ -32,8 +32,7 @@ cudaError_t launch_eval_points(const KeyDev* key, const uint64_t* idx, uint64_t 
                                cudaStream_t st);
 
 // Warp-independent scan (V uint4 per row in 1..32, G keys per warp in 1..4),
-// CTAs of nw warps (warp_cta_warps when the shared memory fits, else half or
-// a quarter).
+// CTAs of nw warps: any number up to warp_cta_warps(G).
 uint32_t warp_slots(int G, uint32_t V, uint32_t M);
 size_t warp_smem_bytes(int G, uint32_t V, uint32_t slots, uint32_t nw);
 bool warp_vt_supported(uint32_t V);

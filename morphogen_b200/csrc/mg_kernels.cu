@@ -473,7 +473,7 @@ __device__ __forceinline__ void xor_out(uint4* out, const uint4 v) {
 // internal nodes and one for leaf pairs (about 25 KB); a third copy runs into
 // the instruction cache: 2^25 x 32 B, 3 keys 2.80 ms with three copies, 2.65
 // with one and a stack round trip per step, 2.61 with two; 2.52 with 20 warps.
-// Bound by integer issue: 89.8% of the issue slots, ALU pipe 90.8%, FMA 84.3%.
+// Bound by integer issue: 90.4% of the issue slots, ALU pipe 91.2%, FMA 86.2%.
 //
 // scan_block_kernel (other row sizes, or several keys per warp): a step's rows
 // are too many for registers.  Its masks, for each of the warp's keys, go to
@@ -727,8 +727,8 @@ __global__ void __launch_bounds__(warp_cta_warps(G) * 32, 1)
   const uint32_t pos = lane % V, r0 = lane / V;
   const bool scans = VT ? true : lane < V * RPL;
   const uint32_t nload = (kRows + RPL - 1) / RPL;  // loads per lane and block
-  // Shared memory: masks of two blocks [nw][2][G][kRows], stacks
-  // [nw][G][slots][32], then the stacks' t masks.
+  // Shared memory: masks of two steps [nw][2][G][kRows], the stages of the row
+  // chunks [nw][CH][32], stacks [nw][G][slots][32], then the stacks' t masks.
   constexpr uint32_t nm = 2u * G * kRows;
   const uint32_t ns = G * p.slots * 32u;
   uint4* const sm4 = reinterpret_cast<uint4*>(smem_raw);
@@ -875,7 +875,7 @@ __global__ void __launch_bounds__(warp_cta_warps(G) * 32, 1)
     // Table row of the warp tile's first leaf (wraps below the first row).
     const uint64_t row0 = (((sg.first >> M) + (uint64_t)tile * 32) << M) - sg.first;
     // A warp tile whose 32 x 2^M rows all lie in the table needs no bounds
-    // checks.  (Depth 1 has no second pair and takes the checked path.)
+    // checks.
     const bool full = row0 < nrows && nrows - row0 >= ((uint64_t)32 << M);
     const uint32_t pairs = 1u << (M - 1);
     for (uint32_t pi = 0; pi < pairs; ++pi) {
@@ -1154,11 +1154,12 @@ __global__ void __launch_bounds__(256) prg_peak_kernel(uint32_t* __restrict__ ou
 
 // ---- host-side launchers --------------------------------------------------
 
-// Launch a kernel that begins with chain_begin(): when the work before it on
-// the stream is such a kernel too, it need not have completed for this one's
-// launch to be processed (programmatic stream serialization; a captured graph
-// gets programmatic edges).  One call of five kernels, 4099 x 32 B: 49.5 us
-// without, 46.0 with; 1300021 x 4 KB pages, launched directly: 998 and 981.
+// Launch a kernel that begins with chain_begin() or chain_wait(): when the work
+// before it on the stream is such a kernel too, it need not have completed for
+// this one's launch to be processed (programmatic stream serialization; a
+// captured graph gets programmatic edges).  One call, 3 keys, without and with:
+// 4099 x 32 B 47.9 and 47.5 us, 1000003 x 48 B 146.0 and 144.3, 1300021 x 4 KB
+// pages 1020 and 1016; calls of milliseconds take the same.
 template <class... P, class... A>
 static cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, uint32_t threads, size_t smem, cudaStream_t st,
                                   A&&... args) {
@@ -1246,18 +1247,23 @@ int scan_occupancy(int G, bool fma, size_t smem) {
 }
 
 // Rows under 2 KB leave the pass bound by its node expansions as much as by
-// memory, and the balanced PRG is faster (3 keys, 10^6 x 528 B: 239 us against
-// 252); wider ones are bound by HBM and its power, where the all-ALU form with
-// fewer instructions wins (1300021 x 4 KB: 887 us against 925).
+// memory, and the balanced PRG is faster: 3 keys, 10^6 x 528 B 239 us against
+// 252 all-ALU.  So it is for the rows of 16 to 512 B that come here with the
+// kernel pinned or from mg_scan_noalloc (pinned, then noalloc): 2^20 x 16 B 180
+// against 193 and 224 against 240, 2^23 x 32 B 900 against 986 and 974 against
+// 1061, 2^20 x 256 B 187 against 198 and 278 against 296, 12 keys over 2^19 x
+// 512 B 351 against 367 and 561 against 590; tables of one wave (20000 rows)
+// take either.  Wider rows are bound by HBM and its power, where the all-ALU
+// form with fewer instructions wins (1300021 x 4 KB: 887 us against 925).
 bool scan_fma(uint32_t V) { return V < 128; }
 
 cudaError_t launch_scan(int G, bool fma, const ScanParams& p, uint32_t grid, size_t smem, cudaStream_t st) {
   const ScanKernel k = scan_kernel_of(G, fma);
   if (!k) return cudaErrorInvalidValue;
-  // Not launched early: its three CTAs per SM would be placed while the
-  // frontier's CTAs still hold some of the SMs' shared memory, unevenly for the
-  // whole pass (3 keys, 10^6 x 528 B: 269 us against 239; 48 keys, 100000 x
-  // 4 KB: 1010 against 885).
+  // Not launched early: beside a kernel that still holds some of the SMs, its
+  // three CTAs per SM are placed unevenly for the whole pass (beside its
+  // frontier, 3 keys, 10^6 x 528 B: 269 us against 239; 48 keys, 100000 x 4 KB:
+  // 1010 against 885).
   k<<<grid, kThreads, smem, st>>>(p);
   return cudaGetLastError();
 }
@@ -1318,8 +1324,9 @@ cudaError_t launch_eval_points(const KeyDev* key, const uint64_t* idx, uint64_t 
 // registers); the block scan keeps a key's root in the first slot too.
 uint32_t warp_slots(int G, uint32_t V, uint32_t M) { const uint32_t top = pair_scan(G, V) ? 2 : 1; return M > top ? M - top : 1; }
 
-// Dynamic shared memory of a warp-kernel CTA of nw warps.  Own-rows scan: a
-// stack per warp.  Block scan: two blocks of masks and a stack per key and warp.
+// Dynamic shared memory of a warp-kernel CTA of nw warps.  Pair scan: a stack
+// per warp, and for 64-B rows a step's masks.  Block scan: a stage per warp, and
+// two steps' masks and a stack per key and warp.
 size_t warp_smem_bytes(int G, uint32_t V, uint32_t slots, uint32_t nw) {
   if (pair_scan(G, V)) return (size_t)nw * 32 * ((V > 2 ? 2 * 16 : 0) + (size_t)slots * 17);
   return (size_t)nw * 32 * ((size_t)block_chunk(V) * 16 + (size_t)G * (2 * kBlockLeaves * 16 + (size_t)slots * 17));
