@@ -176,7 +176,7 @@ int mg_batch_set_keys(mg_batch* batch, const mg_table* const* tables, const uint
                       const size_t* key_lens, uint32_t nkeys);
 /* Pin the launch shape (0 = let the planner choose).  Rows of up to 512 B that
  * are no power of two take any shape: 2^6..2^15 rows and 1..4 keys per item on
- * the warp kernel, the others on the CTA kernel. */
+ * the warp kernel where its frontier has room, the others on the CTA kernel. */
 int mg_batch_set_shape(mg_batch* batch, uint32_t subtree_bits, uint32_t keys_per_cta);
 /* Choose the scan kernel (MG_KERNEL_AUTO by default). */
 int mg_batch_set_kernel(mg_batch* batch, int kind);

@@ -1320,60 +1320,77 @@ int plan_pass(mg_batch* b) {
   // CTA kernel otherwise.  A caller may pin the warp kernel for row sizes that
   // are powers of two only; for the others any tile depth and 8 keys per item
   // may be pinned too, which is the CTA kernel's where the warp kernel has no
-  // such shape (it would refuse the depth or silently take another).
-  const bool warp_shape = (b->eff_S == 0 || (b->eff_S >= 6 && b->eff_S <= kMaxWarpLevels + 5)) &&
-                          (b->eff_G == 0 || mg::warp_g_supported((int)b->eff_G));
-  for (SegPlan& sp : segs) {
-    const uint32_t V = sp.table->row_bytes / 16;
-    const bool ok = mg::warp_vt_supported(V) && sp.d >= 1;
-    const bool pow2 = (V & (V - 1)) == 0;
-    if (b->eff_kind == MG_KERNEL_WARP && (!ok || (b->kind_pref == MG_KERNEL_WARP && !pow2)))
-      return fail(MG_EINVAL, "the warp kernel needs row_bytes in {16..512, powers of two} and d >= 1");
-    sp.warp = ok && b->eff_kind != MG_KERNEL_CTA && (pow2 || warp_shape);
-  }
+  // such shape (it would refuse the depth or silently take another) or its
+  // frontier no room (odd_on_warp).
   // Keys per item: one choice for the CTA kernel, one per row size for the
   // warp kernel (each row size is a launch of its own).
-  uint32_t Vc = 1;
-  size_t nc = 1;
-  std::map<uint32_t, size_t> warp_keys;  // V -> most keys of a segment
+  bool odd_on_warp = false;
   for (const SegPlan& sp : segs) {
     const uint32_t V = sp.table->row_bytes / 16;
-    if (sp.warp) {
-      warp_keys[V] = std::max(warp_keys[V], sp.keys.size());
-    } else {
-      Vc = std::max(Vc, V);
-      nc = std::max(nc, sp.keys.size());
-    }
+    const bool ok = mg::warp_vt_supported(V) && sp.d >= 1, odd = (V & (V - 1)) != 0;
+    if (b->eff_kind == MG_KERNEL_WARP && (!ok || (b->kind_pref == MG_KERNEL_WARP && odd)))
+      return fail(MG_EINVAL, "the warp kernel needs row_bytes in {16..512, powers of two} and d >= 1");
+    odd_on_warp = odd_on_warp || (ok && odd && b->eff_kind != MG_KERNEL_CTA);
   }
-  const int Gc = choose_g(Vc, nc, b->eff_G, false);
-  std::map<uint32_t, int> Gw;
-  for (const auto& vk : warp_keys) Gw[vk.first] = choose_g(vk.first, vk.second, b->eff_G, true);
+  odd_on_warp = odd_on_warp && (b->eff_S == 0 || (b->eff_S >= 6 && b->eff_S <= kMaxWarpLevels + 5)) &&
+                (b->eff_G == 0 || mg::warp_g_supported((int)b->eff_G));
+  int Gc = 1;
+  std::map<uint32_t, int> Gw;  // V -> keys per item
   std::vector<SegPlan> split;
-  for (SegPlan& sp : segs) {
-    const int G = sp.warp ? Gw[sp.table->row_bytes / 16] : Gc;
-    const uint32_t g = (uint32_t)std::min<size_t>((size_t)G, sp.keys.size());
-    const size_t full = sp.keys.size() / g * g;
-    split.push_back(SegPlan{sp.table, sp.d, std::vector<uint32_t>(sp.keys.begin(), sp.keys.begin() + full), g, sp.warp});
-    if (full < sp.keys.size())
-      split.push_back(SegPlan{sp.table, sp.d, std::vector<uint32_t>(sp.keys.begin() + full, sp.keys.end()),
-                              (uint32_t)(sp.keys.size() - full), sp.warp});
-  }
+  auto assign = [&]() {
+    uint32_t Vc = 1;
+    size_t nc = 1;
+    std::map<uint32_t, size_t> warp_keys;  // V -> most keys of a segment
+    for (SegPlan& sp : segs) {
+      const uint32_t V = sp.table->row_bytes / 16;
+      sp.warp = mg::warp_vt_supported(V) && sp.d >= 1 && b->eff_kind != MG_KERNEL_CTA &&
+                ((V & (V - 1)) == 0 || odd_on_warp);
+      if (sp.warp) {
+        warp_keys[V] = std::max(warp_keys[V], sp.keys.size());
+      } else {
+        Vc = std::max(Vc, V);
+        nc = std::max(nc, sp.keys.size());
+      }
+    }
+    Gc = choose_g(Vc, nc, b->eff_G, false);
+    Gw.clear();
+    for (const auto& vk : warp_keys) Gw[vk.first] = choose_g(vk.first, vk.second, b->eff_G, true);
+    split.clear();
+    for (const SegPlan& sp : segs) {
+      const int G = sp.warp ? Gw[sp.table->row_bytes / 16] : Gc;
+      const uint32_t g = (uint32_t)std::min<size_t>((size_t)G, sp.keys.size());
+      const size_t full = sp.keys.size() / g * g;
+      split.push_back(SegPlan{sp.table, sp.d, std::vector<uint32_t>(sp.keys.begin(), sp.keys.begin() + full), g, sp.warp});
+      if (full < sp.keys.size())
+        split.push_back(SegPlan{sp.table, sp.d, std::vector<uint32_t>(sp.keys.begin() + full, sp.keys.end()),
+                                (uint32_t)(sp.keys.size() - full), sp.warp});
+    }
+  };
+  assign();
 
   // The fastest plan, or, where its frontier does not fit the memory or would
   // take more than a quarter of what is free (or than a server may let it have),
-  // the fastest one with at least two,
-  // three, ... depth-first levels per lane (and no frontier for the CTA kernel):
-  // with 10 levels it is a node for 1024 rows and key, where the fastest plan of
-  // a wide-row table has up to one for 8 (17 GB for 48 keys over 340000000 x
-  // 512 B).
+  // the fastest one with at least two, three, ... depth-first levels per lane
+  // (and no frontier for the CTA kernel): with 10 levels it is a node for 1024
+  // rows and key, where the fastest plan of a wide-row table has up to one for 8
+  // (17 GB for 48 keys over 340000000 x 512 B).  When not even that fits, or the
+  // depth is pinned, rows that are no power of two go to the CTA kernel, which
+  // has the same items and can do without a frontier.
   Plan P;
-  for (uint32_t min_levels = 1;; ++min_levels) {
+  for (uint32_t min_levels = 1;;) {
     if (int rc = plan_launches(b, split, Gc, Gw, min_levels, P)) return rc;
     const bool last = min_levels == kMaxWarpLevels;
-    if (!last && scratch_too_large(b, P.need)) continue;
-    const int rc = grow(b, P.need);
-    if (rc == MG_OK) break;
-    if (last || rc != MG_ENOMEM) return rc;
+    if (last || !scratch_too_large(b, P.need)) {
+      const int rc = grow(b, P.need);
+      if (rc == MG_OK) break;
+      if (rc != MG_ENOMEM || (last && !odd_on_warp)) return rc;
+    }
+    if (odd_on_warp && (last || b->eff_S)) {
+      odd_on_warp = false;
+      assign();
+    } else {
+      ++min_levels;
+    }
   }
   std::vector<mg_batch::Launch>& launches = P.launches;
   std::vector<uint32_t>&key_col = P.key_col, &key_bytes = P.key_bytes, &key_slot = P.key_slot;

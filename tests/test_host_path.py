@@ -288,3 +288,46 @@ def test_a_server_splits_a_pass_that_finds_no_memory(fake, fscanner, slots):
     assert err.value.code == N.MG_ENOMEM
     srv.close()
     t.close()
+
+
+@pytest.mark.parametrize("row_bytes", [48, 496])
+@pytest.mark.parametrize("subtree_bits,keys_per_item", [(6, 0), (6, 1), (7, 3), (9, 2)])
+def test_pinned_items_without_room_for_their_frontier_run_on_the_cta_kernel(fake, fscanner, row_bytes, subtree_bits, keys_per_item):
+    # A pinned depth cannot be walked deeper, but the CTA kernel has the same
+    # items and needs no frontier.
+    rows, nkeys = 200_000_003, 24
+    keys = [key(28, i) for i in range(nkeys)]
+    room = 24 * 148 * 32 * row_bytes + (16 << 20)
+    fake.fake_reset(rows * row_bytes + room, 0)
+    t = G.GpuPageMatrix.alloc_empty(fscanner, rows, row_bytes)
+    for spare, kernel in ((0, N.KERNEL_CTA), (1 << 42, N.KERNEL_WARP)):
+        fake.fake_reset(rows * row_bytes + room + spare, 0)
+        ws = fscanner.workspace()
+        ws.set_shape(subtree_bits, keys_per_item)
+        ws.set_keys([t] * nkeys, keys)
+        plan = ws.plan()
+        assert plan["kernel"] == kernel and plan["subtree_bits"] == subtree_bits
+        assert plan["keys_per_cta"] == keys_per_item or not keys_per_item
+        ws.launch()
+        ws.launch(graph=True)
+        assert fake.fake_dead_launches() == 0
+        ws.close()
+    t.close()
+
+
+@pytest.mark.parametrize("rows,row_bytes", [(3_600_000_003, 48), (500_000_001, 336)])
+@pytest.mark.parametrize("shape", [(0, 0), (0, 3)])
+def test_rows_that_are_no_power_of_two_need_no_frontier_when_none_fits(fake, fscanner, rows, row_bytes, shape):
+    nkeys, d = 48, (rows - 1).bit_length()
+    fake.fake_reset(rows * row_bytes + (256 << 20), 0)
+    t = G.GpuPageMatrix.alloc_empty(fscanner, rows, row_bytes)
+    ws = fscanner.workspace()
+    ws.set_shape(*shape)
+    ws.set_keys([t] * nkeys, [key(d, i) for i in range(nkeys)])
+    plan = ws.plan()
+    assert plan["kernel"] == N.KERNEL_CTA and plan["frontier_nodes"] == 0
+    ws.launch()
+    ws.launch(graph=True)
+    assert fake.fake_dead_launches() == 0
+    ws.close()
+    t.close()
